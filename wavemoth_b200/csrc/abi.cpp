@@ -74,15 +74,23 @@ struct ImageRefs {
   int32_t *d_order = nullptr;       // all matrices, largest first (generic kernel over everything)
   int32_t *d_order_slow = nullptr;  // matrices left to the generic kernel by the tensor-core path
   int32_t nslow = 0;
-  // tensor-core path
+  // row groups
   wm::DevGroup *d_groups = nullptr;
   wm::DevGCol *d_gcols = nullptr;
-  wm::DevTileA *d_tiles_a = nullptr;
-  wm::DevTileB *d_tiles_b = nullptr;
   wm::DevRootUnit *d_roots = nullptr;
-  double *d_seeds = nullptr;
+  // FP64 residual path
+  bool direct = false;
+  const wm::DevDirectTileA *d_direct_a[2] = {};
+  int32_t ndirect_a[2] = {};
+  wm::DevDirectTileB *d_direct_b = nullptr;
+  int32_t ndirect_b = 0;
+  double *d_direct_ab = nullptr, *d_direct_scale = nullptr, *d_direct_inj = nullptr;
+  wm::DevDirectCol *d_direct_cols = nullptr;
+  double2 *d_direct_seeds = nullptr;
+  int64_t *d_direct_tile_seeds = nullptr;
   // split-precision path
   bool split = false;
+  double *d_seeds = nullptr;
   wm::DevSplitGroup *d_sgroups = nullptr;
   wm::DevSplitTileA *d_stiles_a = nullptr;
   wm::DevSplitTileB *d_stiles_b = nullptr;
@@ -320,24 +328,39 @@ wm::FastParams fast_params(wavemoth_plan P) {
   f.i32 = P->d_i32;
   f.groups = P->d_groups;
   f.gcols = P->d_gcols;
-  f.tiles_a = P->d_tiles_a;
-  f.tiles_b = P->d_tiles_b;
   f.roots = P->d_roots;
-  f.seeds = P->d_seeds;
   f.ngroups = (int32_t)G.groups.size();
   f.ngcols = (int64_t)G.gcols.size();
-  f.ntiles_a = (int32_t)G.tiles_a.size();
-  f.ntiles_b = (int32_t)G.tiles_b.size();
   f.nroots = (int32_t)G.roots.size();
   f.max_root_k = G.max_root_k;
   f.max_root_n = G.max_root_n;
-  f.lmax = P->lmax;
   f.nvecs = P->nvecs;
-  f.ni = P->ni;
   f.q_mstride = P->nvecs;
   f.q_rstride = 2LL * shard_mcount(P) * P->nvecs;
   f.xbuf = P->d_xbuf;
   return f;
+}
+
+wm::DirectParams direct_params(wavemoth_plan P) {
+  wm::DirectParams d{};
+  d.mats = P->d_mats;
+  d.groups = P->d_groups;
+  d.cols = P->d_direct_cols;
+  d.inj = P->d_direct_inj;
+  d.ab = reinterpret_cast<const double2 *>(P->d_direct_ab);
+  d.scale = P->d_direct_scale;
+  d.seeds = P->d_direct_seeds;
+  d.tile_seeds = P->d_direct_tile_seeds;
+  d.tiles_b = P->d_direct_b;
+  d.ntiles_b = P->ndirect_b;
+  d.ngroups = (int32_t)P->img->prog.groups.size();
+  d.ngcols = (int64_t)P->img->prog.gcols.size();
+  d.lmax = P->lmax;
+  d.nvecs = P->nvecs;
+  d.q_mstride = P->nvecs;
+  d.q_rstride = 2LL * shard_mcount(P) * P->nvecs;
+  d.xbuf = P->d_xbuf;
+  return d;
 }
 
 wm::SplitParams split_params(wavemoth_plan P) {
@@ -432,10 +455,27 @@ int build_image(DeviceImage &I, int nside, int mmax, unsigned flags) {
   }
   rc = rc ? rc : upload(A, &I.d_groups, G.groups, "groups");
   rc = rc ? rc : upload(A, &I.d_gcols, G.gcols, "group columns");
-  rc = rc ? rc : upload(A, &I.d_tiles_a, G.tiles_a, "alm2map tiles");
-  rc = rc ? rc : upload(A, &I.d_tiles_b, G.tiles_b, "map2alm tiles");
   rc = rc ? rc : upload(A, &I.d_roots, G.roots, "roots");
-  rc = rc ? rc : A.alloc(&I.d_seeds, (size_t)std::max<int64_t>(G.nseeds, 1), "recurrence seeds");
+  I.split = (flags & WAVEMOTH_PRECISION_SPLIT) != 0;
+  I.direct = !I.split;
+  if (I.direct) {
+    const size_t nc = G.gcols.size();
+    for (int w = 0; w < 2; ++w) {
+      wm::DevDirectTileA *tiles = nullptr;
+      rc = rc ? rc : upload(A, &tiles, G.direct_a[w], "alm2map tiles");
+      I.d_direct_a[w] = tiles;
+      I.ndirect_a[w] = (int32_t)G.direct_a[w].size();
+    }
+    rc = rc ? rc : upload(A, &I.d_direct_b, G.direct_b, "map2alm tiles");
+    I.ndirect_b = (int32_t)G.direct_b.size();
+    rc = rc ? rc : upload(A, &I.d_direct_tile_seeds, G.direct_tile_seeds, "seed tables");
+    rc = rc ? rc : upload(A, &I.d_direct_ab, G.direct_ab, "row coefficients");
+    rc = rc ? rc : upload(A, &I.d_direct_scale, G.direct_scale, "row scales");
+    rc = rc ? rc : A.alloc(&I.d_direct_cols, nc, "column table");
+    rc = rc ? rc : A.alloc(&I.d_direct_inj, nc * wm::kDirectInj, "column first values");
+    rc = rc ? rc : A.alloc(&I.d_direct_seeds, (size_t)G.direct_seeds, "segment seeds");
+  }
+  if (I.split) rc = rc ? rc : A.alloc(&I.d_seeds, (size_t)std::max<int64_t>(G.nseeds, 1), "recurrence seeds");
   I.program_bytes = A.bytes;
   {
     RingTable RT = ring_table(nside, 1, mmax);
@@ -449,7 +489,6 @@ int build_image(DeviceImage &I, int nside, int mmax, unsigned flags) {
     rc = rc ? rc : A.alloc(&I.d_ring_aux, (size_t)std::max<int64_t>(2 * RT.aux_cplx, 2), "Bluestein chirps");
     rc = rc ? rc : A.alloc(&I.d_phases, (size_t)(2 * nside) * (wm::kRingPhaseLo + RT.nphase_hi), "phase tables");
   }
-  I.split = (flags & WAVEMOTH_PRECISION_SPLIT) != 0;
   if (I.split) {
     rc = rc ? rc : upload(A, &I.d_sgroups, G.sgroups, "split groups");
     rc = rc ? rc : upload(A, &I.d_stiles_a, G.stiles_a, "split alm2map tiles");
@@ -500,7 +539,15 @@ int init_image(wavemoth_plan P) {
                                           P->d_ring_aux, P->d_phases, P->stream), "ring setup launch");
     if (!rc) rc = cuda_check(cudaStreamSynchronize(P->stream), "ring setup");
   }
-  if (!rc && G.nseeds > 0) {
+  if (!rc && P->direct && !G.gcols.empty()) {
+    rc = cuda_check(cudaMemsetAsync(P->d_direct_seeds, 0, std::max<int64_t>(G.direct_seeds, 1) * sizeof(double2),
+                                    P->stream), "segment seeds");
+    if (!rc)
+      rc = cuda_check(wm::launch_direct_setup(direct_params(P), P->d_gcols, P->d_f64, P->d_direct_cols,
+                                              P->d_direct_inj, P->d_direct_seeds, P->stream), "column setup launch");
+    if (!rc) rc = cuda_check(cudaStreamSynchronize(P->stream), "column setup");
+  }
+  if (!rc && P->split && G.nseeds > 0) {
     wm::FastParams fp = fast_params(P);
     fp.seeds_out = P->d_seeds;
     rc = cuda_check(wm::launch_seeds(fp, P->stream), "seed kernel launch");
@@ -536,7 +583,9 @@ int init_image(wavemoth_plan P) {
     G.f64.clear(); G.f64.shrink_to_fit();
     G.i32.clear(); G.i32.shrink_to_fit();
     G.gcols.clear(); G.gcols.shrink_to_fit();
-    G.tiles_a.shrink_to_fit();
+    G.direct_ab.clear(); G.direct_ab.shrink_to_fit();
+    G.direct_scale.clear(); G.direct_scale.shrink_to_fit();
+    G.direct_tile_seeds.clear(); G.direct_tile_seeds.shrink_to_fit();
   }
   return rc;
 }
@@ -987,27 +1036,49 @@ int run_split(wavemoth_plan P, bool alm2map, const double *alm_in, double *alm_o
   return 0;
 }
 
+// FP64 path: residual products, and the interpolation levels of depth-1
+// matrices after (alm2map) or before them (map2alm).
+int run_direct(wavemoth_plan P, bool alm2map, const double *alm_in, double *alm_out, const double *q_in,
+               double *q_out, cudaStream_t st) {
+  const auto &G = P->img->prog;
+  const int nr = (int)G.roots.size(), cap = P->grid_cap > 0 ? 4 * plan_sms(P) : 0;
+  int rc = 0;
+  auto levels = [&]() {
+    if (rc || !nr) return;
+    wm::FastParams f = fast_params(P);
+    f.q_in = q_in;
+    f.q = q_out;
+    rc = cuda_check(wm::launch_fast(alm2map ? 1 : 2, f, fast_grid(P, nr), st), "level launch");
+    P->kernel_launches++;
+  };
+  wm::DirectParams d = direct_params(P);
+  d.alm_in = alm_in;
+  d.alm_out = alm_out;
+  d.q_in = q_in;
+  d.q = q_out;
+  if (alm2map) {
+    d.aligned = (((uintptr_t)q_out | (uintptr_t)alm_in) & 15) == 0;
+    rc = cuda_check(wm::launch_direct_a2m(d, P->d_direct_a, P->ndirect_a, plan_sms(P), cap, st),
+                    "alm2map residual launch");
+    P->kernel_launches += P->ndirect_a[0] > 0;
+    levels();
+  } else {
+    levels();
+    if (!rc) rc = cuda_check(wm::launch_direct_m2a(d, cap, st), "map2alm residual launch");
+    P->kernel_launches += d.ntiles_b > 0;
+  }
+  return rc;
+}
+
 int run_legendre(wavemoth_plan P, bool alm2map, const double *alm_in, double *alm_out,
                  const double *q_in, double *q_out, cudaStream_t st) {
   const auto &G = P->img->prog;
   int sp = span_begin(P, alm2map ? 0 : 1, st);
   int rc = 0;
-  wm::FastParams f = fast_params(P);
-  f.alm_in = alm_in;
-  f.alm_out = alm_out;
-  f.q_in = q_in;
-  f.q = q_out;
-  const int nta = (int)G.tiles_a.size(), ntb = (int)G.tiles_b.size(), nr = (int)G.roots.size();
   if (P->split) {
     rc = run_split(P, alm2map, alm_in, alm_out, q_in, q_out, st);
-  } else if (alm2map) {
-    if (nta) rc = cuda_check(wm::launch_fast(0, f, fast_grid(P, nta), st), "alm2map residual launch");
-    if (!rc && nr) rc = cuda_check(wm::launch_fast(1, f, fast_grid(P, nr), st), "alm2map level launch");
-    P->kernel_launches += (nta > 0) + (nr > 0);
   } else {
-    if (nr) rc = cuda_check(wm::launch_fast(2, f, fast_grid(P, nr), st), "map2alm level launch");
-    if (!rc && ntb) rc = cuda_check(wm::launch_fast(3, f, fast_grid(P, ntb), st), "map2alm residual launch");
-    P->kernel_launches += (ntb > 0) + (nr > 0);
+    rc = run_direct(P, alm2map, alm_in, alm_out, q_in, q_out, st);
   }
   if (!rc && P->nslow > 0) {
     wm::LegendreParams p = legendre_params(P);

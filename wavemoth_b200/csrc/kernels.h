@@ -42,28 +42,57 @@ struct FastParams {
   const int32_t *i32;
   const DevGroup *groups;
   const DevGCol *gcols;
-  const DevTileA *tiles_a;
-  const DevTileB *tiles_b;
   const DevRootUnit *roots;
-  const double *seeds;     // read by the map2alm residual kernel
-  double *seeds_out;       // written by the seed kernel (plan creation)
+  double *seeds_out;       // written by the seed kernel (plan creation, split images)
   int32_t ngroups;
   int64_t ngcols;
-  int32_t ntiles_a, ntiles_b, nroots;
+  int32_t nroots;
   int32_t max_root_k, max_root_n;
-  int32_t lmax, nvecs, ni;
-  const double *alm_in;    // alm2map input
-  double *alm_out;         // map2alm output
+  int32_t nvecs;
   const double *q_in;      // map2alm input q~
   double *q;               // alm2map output q
   int64_t q_mstride, q_rstride;  // q row of (m, parity, ring): (2m + parity) q_mstride + ring q_rstride
   double *xbuf;            // depth-1 root blocks: X buffer (xrows x nvecs)
 };
 
-// which: 0 alm2map residual, 1 alm2map level, 2 map2alm level, 3 map2alm residual
+// which: 1 alm2map level, 2 map2alm level
 cudaError_t launch_fast(int which, const FastParams &prm, int grid, cudaStream_t st);
 cudaError_t launch_seeds(const FastParams &prm, cudaStream_t st);
 int fast_vector_tiles(int nvecs);
+
+// Residual products on the FP64 units (legendre_direct.cu).
+struct DirectParams {
+  const DevMatrix *mats;
+  const DevGroup *groups;
+  const DevDirectCol *cols;     // per group column
+  const double *inj;            // kDirectInj stored first values of y per group column
+  const double2 *ab;            // (A, B) per group row
+  const double *scale;          // s per group row
+  const double2 *seeds;         // segment seeds (DevDirectTileB)
+  const int64_t *tile_seeds;    // first seed of every row tile of every group (DevGroup::tile_b)
+  const DevDirectTileA *tiles_a;
+  const DevDirectTileB *tiles_b;
+  int32_t ntiles_a, ntiles_b;
+  int32_t ngroups;
+  int64_t ngcols;
+  int32_t lmax, nvecs;
+  const double *alm_in;
+  double *alm_out;
+  const double *q_in;
+  double *q;
+  int64_t q_mstride, q_rstride;
+  double *xbuf;
+  int32_t aligned;              // the alm and q are 16-byte aligned
+};
+
+// max_ctas > 0 bounds the grid (the units are then walked by fewer CTAs);
+// tiles: the alm2map units of kDirectTile and of 2 kDirectTile columns.
+cudaError_t launch_direct_a2m(DirectParams prm, const DevDirectTileA *const (&tiles)[2], const int32_t (&ntiles)[2],
+                              int sms, int max_ctas, cudaStream_t st);
+cudaError_t launch_direct_m2a(const DirectParams &prm, int max_ctas, cudaStream_t st);
+// Plan creation: cols, inj and seeds (zeroed by the caller) of every group column.
+cudaError_t launch_direct_setup(const DirectParams &prm, const DevGCol *gcols, const double *f64, DevDirectCol *cols,
+                                double *inj, double2 *seeds, cudaStream_t st);
 
 // Split-precision residual path (legendre_split.cu).
 struct SplitParams {

@@ -76,7 +76,7 @@ struct DevMatrix {
   int32_t pad2;
 };
 
-// ---- tensor-core (DMMA) path for matrices of tree depth 0 or 1 ----
+// ---- row groups of the matrices of tree depth 0 or 1 ----
 //
 // A "row group" is the set of residual blocks that share one range of matrix
 // rows: the single block of a depth-0 matrix, or the T (respectively B)
@@ -92,6 +92,9 @@ struct DevGroup {
   int64_t seeds;      // index (in doubles) of the group's seeds: ncols x nchunks x 2
   int32_t nchunks;    // seed chunks of kSeedRows rows
   int32_t in_q;       // 1: the columns are rows of q (depth 0); 0: rows of the X buffer
+  int64_t coef;       // FP64 path: index of the group's first row coefficient
+  int32_t seg;        // FP64 path: rows of a map2alm segment
+  int32_t tile_b;     // FP64 path: index of the group's first map2alm row tile
 };
 
 struct DevGCol {
@@ -105,20 +108,35 @@ struct DevGCol {
   int64_t aux;        // f64 offset of the block's recurrence coefficients
 };
 
-struct DevTileA {     // alm2map residual unit: <= 64 consecutive group columns
+// Residual products on the FP64 units (legendre_direct.cu).  P_r = s_r y_r,
+// y_r = (x^2 A_r + B_r) y_{r-1} - y_{r-2}: per group row (A, B) and s, per
+// group column its x^2, first active row and stored first values of y.
+struct DevDirectCol {
+  double x2;
+  int32_t start;      // first active row (group coordinates); INT_MAX: none
+  int32_t row;        // row in q or in the matrix's X buffer, with kDirectDense
+};
+constexpr int32_t kDirectDense = 1 << 30;  // DevDirectCol::row: every active row is stored
+constexpr int kDirectInj = 4;              // stored y values of a column (dense columns have at most 4 active rows)
+constexpr int kDirectSeg = 16;             // most rows of a segment (a lane's share of a map2alm row tile), a multiple of 4
+constexpr int kDirectTile = 128;           // columns of a narrow alm2map unit (a wide one has twice as many)
+
+struct DevDirectTileA {  // alm2map unit: `ncols` consecutive group columns, rows from kstart
   int32_t group, col0, ncols, kstart;
 };
 
-struct DevTileB {     // map2alm residual unit: <= kPushRows consecutive group rows
-  int32_t group, row0, nrows, chunk;   // chunk: seed chunk of row0
+struct DevDirectTileB {  // map2alm unit: 8 segments of `seg` rows from row0, the first nact columns
+  int32_t group, row0, seg, nact;
+  int32_t nfull, pad;    // the first nfull are recurrence columns that start at row0 or before
+  int64_t seeds;         // double2 index: y at rows (j, j + 1), j the first row of segment g, of column
+                         // c at 32 (c / 4) + 4 g + c % 4 (zero where j precedes the column's start)
 };
 
 struct DevRootUnit {  // depth-1 level unit: one root's interpolation pair
   int32_t matrix, pair;
 };
 
-constexpr int kPushRows = 32;   // rows of a map2alm residual unit (FP64 tensor-core path)
-constexpr int kSeedRows = 16;   // spacing of the recurrence seeds (P at rows s, s + 1)
+constexpr int kSeedRows = 16;   // split path: spacing of the recurrence seeds (P at rows s, s + 1)
 
 // ---- split-precision residual path (sliced int8 operands, tcgen05) ----
 //

@@ -755,11 +755,83 @@ static void build_split_tables(HostProgram &P) {
   build_stream_tables(P);
 }
 
+// Scaled recurrence of rows [rs, re) of matrix M (group g: every block of a
+// depth-0 matrix, the T or the B blocks of a depth-1 matrix): P_r = s_r y_r,
+// y_r = (x^2 A_r + B_r) y_{r-1} - y_{r-2} from the stored
+// P_r = (x^2 + alpha) beta P_{r-1} + gamma P_{r-2}.  Every block stores the
+// coefficients of its own rows; false when two blocks disagree or the scale
+// cannot be formed (gamma >= 0), which leaves the matrix to the generic
+// kernels.
+static bool direct_coefficients(const HostProgram &P, const DevMatrix &M, int g, int32_t rs, int32_t re,
+                                std::vector<double> &ab, std::vector<double> &scale) {
+  const int32_t R = re - rs;
+  ab.assign(2 * (size_t)R, 0.0);
+  scale.assign((size_t)R, 1.0);
+  const double *aux = nullptr;  // coefficients of rows boff + 2 .. R - 1 of the widest block
+  int32_t boff = R;
+  for (int pass = 0; pass < 2; ++pass)
+    for (int b = M.dblock_begin; b < M.dblock_end; ++b) {
+      if (M.nlevels == 1 && (b - M.dblock_begin) % 2 != g) continue;
+      const DevDBlock &D = P.dblocks[b];
+      bool recurrence = false;
+      for (int32_t s = D.strip_begin; s < D.strip_end; ++s) recurrence = recurrence || P.strips[s].kind == 1;
+      if (!recurrence) continue;
+      const int32_t off = D.row_start - rs;
+      const double *x = P.f64.data() + D.aux;
+      if (pass == 0) {
+        if (off < boff) {
+          boff = off;
+          aux = x;
+        }
+      } else if (memcmp(x, aux + 3 * (int64_t)(off - boff), 3 * (size_t)(D.nrows - 2) * sizeof(double)) != 0) {
+        return false;
+      }
+    }
+  for (int32_t r = boff + 2; r < R; ++r) {
+    const double *c = aux + 3 * (int64_t)(r - boff - 2);
+    const double s = -c[2] * scale[r - 2], A = c[1] * scale[r - 1] / s, B = c[0] * A;
+    if (!(s > 0.0) || !std::isfinite(s) || !std::isfinite(A) || !std::isfinite(B)) return false;
+    scale[r] = s;
+    ab[2 * (size_t)r] = A;
+    ab[2 * (size_t)r + 1] = B;
+  }
+  return true;
+}
+
+// Work units of group `gi` on the FP64 units: column tiles (alm2map), row
+// tiles of 8 segments of at most kDirectSeg rows (map2alm; the columns that start before the tile's end are a prefix).
+static void direct_tiles(HostProgram &P, DevGroup &G, int32_t gi) {
+  const DevGCol *cols = P.gcols.data() + G.cols;
+  for (int32_t w = 0; w < 2; ++w)
+    for (int32_t c0 = 0; c0 < G.ncols; c0 += kDirectTile << w)
+      P.direct_a[w].push_back(
+          DevDirectTileA{gi, c0, std::min(kDirectTile << w, G.ncols - c0), std::min(cols[c0].start, G.nrows)});
+  // segment length, a multiple of four: rows padded to whole tiles, and
+  // per segment the seeds to read, worth about three rows
+  auto cost = [&](int32_t seg) { return (double)((G.nrows + 8 * seg - 1) / (8 * seg)) * (seg + 3); };
+  G.seg = kDirectSeg;
+  for (int32_t seg = kDirectSeg - 4; seg >= 4; seg -= 4)
+    if (cost(seg) < cost(G.seg)) G.seg = seg;
+  G.tile_b = (int32_t)P.direct_tile_seeds.size();
+  int32_t nact = 0, nfull = 0;
+  for (int32_t r0 = 0; r0 < G.nrows; r0 += 8 * G.seg) {
+    while (nfull < G.ncols && cols[nfull].start <= r0 && cols[nfull].kind == 1) ++nfull;
+    while (nact < G.ncols && cols[nact].start < std::min(G.nrows, r0 + 8 * G.seg)) ++nact;
+    P.direct_b.push_back(DevDirectTileB{gi, r0, G.seg, nact, nfull, 0, P.direct_seeds});
+    P.direct_tile_seeds.push_back(P.direct_seeds);
+    P.direct_seeds += 32 * (int64_t)((nact + 3) / 4);
+  }
+}
+
 bool build_fast_path(HostProgram &P, std::string &err) {
   P.groups.clear();
   P.gcols.clear();
-  P.tiles_a.clear();
-  P.tiles_b.clear();
+  P.direct_ab.clear();
+  P.direct_scale.clear();
+  for (auto &t : P.direct_a) t.clear();
+  P.direct_b.clear();
+  P.direct_tile_seeds.clear();
+  P.direct_seeds = 0;
   P.roots.clear();
   P.slow_mats.clear();
   P.nseeds = 0;
@@ -772,7 +844,7 @@ bool build_fast_path(HostProgram &P, std::string &err) {
     M.xrow = -1;
     if (P.shard_m1 >= 0 && (M.m < P.shard_m0 || M.m >= P.shard_m1)) continue;  // another shard's
     const int nblk = M.dblock_end - M.dblock_begin;
-    bool ok = M.nk > 0 && (M.nlevels == 0 || M.nlevels == 1);
+    bool ok = M.nlevels == 0 || M.nlevels == 1;
     if (ok && M.nlevels == 0) ok = (nblk == 1);
     if (ok && M.nlevels == 1) {
       ok = (nblk % 2 == 0);
@@ -791,6 +863,9 @@ bool build_fast_path(HostProgram &P, std::string &err) {
         ok = D.row_start >= rg.first && D.row_start + D.nrows == rg.second;
       }
     }
+    std::vector<double> ab[2], scale[2];
+    for (size_t g = 0; ok && g < ranges.size(); ++g)
+      ok = direct_coefficients(P, M, (int)g, ranges[g].first, ranges[g].second, ab[g], scale[g]);
     if (!ok) {
       P.slow_mats.push_back((int32_t)mi);
       continue;
@@ -854,21 +929,21 @@ bool build_fast_path(HostProgram &P, std::string &err) {
       G.nchunks = (G.nrows + kSeedRows - 1) / kSeedRows;
       G.seeds = P.nseeds;
       P.nseeds += 2LL * G.ncols * G.nchunks;
-      const int32_t gi = (int32_t)P.groups.size();
+      G.coef = (int64_t)P.direct_scale.size();
+      P.direct_ab.insert(P.direct_ab.end(), ab[g].begin(), ab[g].end());
+      P.direct_scale.insert(P.direct_scale.end(), scale[g].begin(), scale[g].end());
+      direct_tiles(P, G, (int32_t)P.groups.size());
       P.groups.push_back(G);
-      const int32_t ntiles = (G.ncols + 255) / 256;
-      const int32_t width = ntiles ? ((G.ncols + ntiles - 1) / ntiles + 7) & ~7 : 8;
-      for (int32_t c0 = 0; c0 < G.ncols; c0 += width) {
-        DevTileA T{gi, c0, std::min(width, G.ncols - c0), G.nrows};
-        for (int32_t c = c0; c < c0 + T.ncols; ++c)
-          T.kstart = std::min(T.kstart, P.gcols[G.cols + c].start);
-        T.kstart &= ~3;
-        P.tiles_a.push_back(T);
-      }
-      for (int32_t r0 = 0; r0 < G.nrows; r0 += kPushRows)
-        P.tiles_b.push_back(DevTileB{gi, r0, std::min(kPushRows, G.nrows - r0), r0 / kSeedRows});
     }
   }
+  auto rows_left = [&](const DevDirectTileA &t) { return P.groups[t.group].nrows - t.kstart; };
+  for (auto &t : P.direct_a)
+    std::stable_sort(t.begin(), t.end(), [&](const DevDirectTileA &a, const DevDirectTileA &b) {
+      return rows_left(a) > rows_left(b);
+    });
+  std::stable_sort(P.direct_b.begin(), P.direct_b.end(), [](const DevDirectTileB &a, const DevDirectTileB &b) {
+    return (int64_t)a.nact * a.seg > (int64_t)b.nact * b.seg;
+  });
   build_split_tables(P);
   return true;
 }

@@ -22,11 +22,15 @@ struct HostProgram {
   std::vector<double> f64;
   std::vector<int32_t> i32;
   std::vector<int64_t> element_count;   // header element_count per (2m + odd)
-  // tensor-core path tables (see plan.h)
+  // row groups and their tables (see plan.h)
   std::vector<DevGroup> groups;
   std::vector<DevGCol> gcols;
-  std::vector<DevTileA> tiles_a;
-  std::vector<DevTileB> tiles_b;
+  std::vector<double> direct_ab;        // FP64 path: (A, B) per group row
+  std::vector<double> direct_scale;     // and s
+  std::vector<DevDirectTileA> direct_a[2];              // alm2map units (narrow, wide), largest first
+  std::vector<DevDirectTileB> direct_b;                 // map2alm units, largest first
+  std::vector<int64_t> direct_tile_seeds;               // seeds of every group's row tiles (DevGroup::tile_b)
+  int64_t direct_seeds = 0;             // double2 entries of all seeds
   std::vector<DevRootUnit> roots;
   std::vector<int32_t> slow_mats;       // matrices left to the generic kernels
   int64_t nseeds = 0;                   // doubles of recurrence seeds
@@ -82,7 +86,8 @@ inline int64_t q_row(const HostProgram &P, int m, int odd, int64_t ring) {
 // Streamed split GEMM launches.
 enum : int { kStreamResA2M = 0, kStreamResM2A = 1, kStreamLevelA2M = 2, kStreamLevelM2A = 3 };
 
-// Builds the tensor-core path tables for matrices of depth 0 and 1.
+// Builds the row groups and the tables of both residual paths for matrices
+// of depth 0 and 1.
 bool build_fast_path(HostProgram &P, std::string &err);
 
 // One serialized butterfly matrix (the per-matrix layout of a rev1 file,
