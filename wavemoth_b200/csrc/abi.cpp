@@ -952,10 +952,6 @@ void span_end(wavemoth_plan P, int idx, cudaStream_t st) {
 // scheduler's cap, else all)
 int plan_sms(wavemoth_plan P) { return P->grid_cap > 0 ? std::min(P->grid_cap, P->sm_count) : P->sm_count; }
 
-int fast_grid(wavemoth_plan P, int units) {
-  return std::max(1, std::min(units, 4 * plan_sms(P)));
-}
-
 // Split-precision residual products, kSplitN vectors per pass: operand
 // slices of the pass, then the tensor-core GEMM of every group tile.
 // Launch description of streamed split GEMM k (wm::kStream*).
@@ -1048,7 +1044,7 @@ int run_direct(wavemoth_plan P, bool alm2map, const double *alm_in, double *alm_
     wm::FastParams f = fast_params(P);
     f.q_in = q_in;
     f.q = q_out;
-    rc = cuda_check(wm::launch_fast(alm2map ? 1 : 2, f, fast_grid(P, nr), st), "level launch");
+    rc = cuda_check(wm::launch_level(alm2map, f, cap, st), "level launch");
     P->kernel_launches++;
   };
   wm::DirectParams d = direct_params(P);

@@ -55,10 +55,10 @@ struct FastParams {
   double *xbuf;            // depth-1 root blocks: X buffer (xrows x nvecs)
 };
 
-// which: 1 alm2map level, 2 map2alm level
-cudaError_t launch_fast(int which, const FastParams &prm, int grid, cudaStream_t st);
+// Interpolation levels of the depth-1 matrices (legendre_mma.cu); max_ctas > 0
+// bounds the grid.
+cudaError_t launch_level(bool alm2map, const FastParams &prm, int max_ctas, cudaStream_t st);
 cudaError_t launch_seeds(const FastParams &prm, cudaStream_t st);
-int fast_vector_tiles(int nvecs);
 
 // Residual products on the FP64 units (legendre_direct.cu).
 struct DirectParams {

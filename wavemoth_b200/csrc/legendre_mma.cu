@@ -6,6 +6,7 @@
 // where W[z][s] is the (n x k) matrix of one interpolation block with its
 // filter folded in: row z is the unit vector e_s' if z is skeleton column s'
 // (filter 0), else column c(z) of the interpolant (src/butterfly.c.in:222-235).
+// The unit vectors' rows are copies; only the interpolants are multiplied.
 //
 // Fragment layout of mma.m8n8k4 .f64 (lane = 4 g + t): A (8x4, row) element
 // (g, t); B (4x8, col) element (t, g); C/D (8x8) elements (g, 2t) and (g, 2t+1).
@@ -14,7 +15,10 @@
 // are bitwise reproducible.  k_seeds stores P at every kSeedRows-th row of
 // every column once per split plan (legendre_split.cu slices P from them).
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <stdint.h>
+
+#include <algorithm>
 
 #include "kernels.h"
 #include "plan.h"
@@ -38,140 +42,149 @@ __device__ __forceinline__ double rec_step(const double *f64, const DevGCol &C, 
   return (x2 + ab[0]) * ab[1] * pc + ab[2] * pp;
 }
 
-// W[z][s] of one interpolation block (k skeleton columns, n rows z).
-__device__ __forceinline__ double w_elem(const int32_t *map, const double *ip_t, int n, int k, int z,
-                                         int s) {
-  if (z >= n || s >= k) return 0.0;
-  const int mt = map[z];
-  if (mt < 0) return (s == -mt - 1) ? 1.0 : 0.0;
-  return ip_t[mt + (int64_t)s * (n - k)];
-}
-
-// ------------------------------------------------------------------------
-// alm2map level: one unit = one depth-1 root; q rows = W_T X_T + W_B X_B.
-// ------------------------------------------------------------------------
+// Row stride (doubles) of a staged operand of NT vector tiles: the four rows
+// of a B fragment start in different halves of the 128 bytes of banks.
 template <int NT>
-__global__ void __launch_bounds__(kThr) k_a2m_level(FastParams p) {
-  constexpr int VT = 8 * NT;
-  constexpr int VP = VT + 8;
-  extern __shared__ double xs[];  // (kT + kB rounded to 4) x VP
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int g4 = lane >> 2, t4 = lane & 3;
-  for (int unit = blockIdx.x; unit < p.nroots; unit += gridDim.x) {
-    const DevRootUnit U = p.roots[unit];
-    const DevMatrix M = p.mats[U.matrix];
-    const DevPair P = p.pairs[U.pair];
-    const int K = P.kT + P.kB, K4 = (K + 3) & ~3;
-    const double *X = p.xbuf + M.xrow * p.nvecs;
-    double *qm = p.q + (int64_t)(2 * M.m + M.odd) * p.q_mstride;
-    const int32_t *mapT = p.i32 + P.mapT, *mapB = p.i32 + P.mapB;
-    const double *ipT = p.f64 + P.ipT_t, *ipB = p.f64 + P.ipB_t;
-    for (int v0 = 0; v0 < p.nvecs; v0 += VT) {
-      const int vn = min(VT, p.nvecs - v0);
-      __syncthreads();
-      for (int idx = threadIdx.x; idx < K4 * VT; idx += kThr) {
-        const int s = idx / VT, v = idx % VT;
-        double val = 0.0;
-        if (s < K && v < vn) {
-          const int row = s < P.kT ? P.inT + s : P.inB + (s - P.kT);
-          val = X[(int64_t)row * p.nvecs + v0 + v];
-        }
-        xs[s * VP + v] = val;
-      }
-      __syncthreads();
-      for (int z0 = 0; z0 < P.n; z0 += 128) {
-        double acc[2][NT][2];
+constexpr int kLevelPitch = NT == 1 ? 8 : 8 * NT + 8;
+
+// D = A x B for rows 8 mt .. + 7 of one interpolation block: A(row, j) =
+// a[row + j lda] (rows beyond `rows` repeat the last one and are not stored),
+// B(j, v) the staged row b(j).  Eight steps of A are in flight at once.
+template <int NT, class RowF>
+__device__ __forceinline__ void level_tile(const double *a, int lda, int rows, int depth, int mt, RowF b,
+                                           double (&acc)[NT][2]) {
+  const int lane = threadIdx.x & 31, g4 = lane >> 2, t4 = lane & 3;
+  const double *ap = a + min(8 * mt + g4, rows - 1);
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+  for (int nt = 0; nt < NT; ++nt) acc[nt][0] = acc[nt][1] = 0.0;
+  for (int j0 = 0; j0 < depth; j0 += 32) {
+    double x[8];
 #pragma unroll
-          for (int nt = 0; nt < NT; ++nt) acc[i][nt][0] = acc[i][nt][1] = 0.0;
-        for (int ks = 0; ks < K4 / 4; ++ks) {
-          const int s = 4 * ks + t4;
-          double a[2];
+    for (int i = 0; i < 8; ++i) {
+      const int j = j0 + 4 * i + t4;
+      x[i] = j < depth ? ap[(int64_t)j * lda] : 0.0;
+    }
 #pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            const int z = z0 + 16 * warp + 8 * i + g4;
-            a[i] = s < P.kT ? w_elem(mapT, ipT, P.n, P.kT, z, s)
-                            : w_elem(mapB, ipB, P.n, P.kB, z, s - P.kT);
-          }
+    for (int i = 0; i < 8; ++i) {
+      if (j0 + 4 * i >= depth) break;
+      const double *row = b(min(j0 + 4 * i + t4, depth - 1)) + g4;
 #pragma unroll
-          for (int nt = 0; nt < NT; ++nt) {
-            const double b = xs[s * VP + 8 * nt + g4];
-            dmma(acc[0][nt], a[0], b);
-            dmma(acc[1][nt], a[1], b);
-          }
-        }
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          const int z = z0 + 16 * warp + 8 * i + g4;
-          if (z >= P.n) continue;
-          double *dst = qm + (int64_t)(P.out_left + z) * p.q_rstride + v0;
-#pragma unroll
-          for (int nt = 0; nt < NT; ++nt) {
-            const int v = 8 * nt + 2 * t4;
-            if (v < vn) dst[v] = acc[i][nt][0];
-            if (v + 1 < vn) dst[v + 1] = acc[i][nt][1];
-          }
-        }
-      }
+      for (int nt = 0; nt < NT; ++nt) dmma(acc[nt], x[i], row[8 * nt]);
     }
   }
 }
 
 // ------------------------------------------------------------------------
-// map2alm level: one unit = one depth-1 root; X_T = W_T^T q~, X_B = W_B^T q~.
+// alm2map level: one unit = one depth-1 root and 8 NT vectors.  q rows are the
+// sum of the T and the B block's rows; a block's k skeleton rows are its X
+// rows, its other n - k the interpolant (rows of the stored transpose) times
+// X.  Interpolant rows are taken in storage order, so that A fragments are
+// read from global memory as 64-byte runs without a look-up, and put in
+// place through the row permutation when a tile is done.
+//
+// Bound: the latency of a root's small products (about 64 x 64 per block), so
+// several CTAs per SM.  Reading W[z][s] through the row map element by element
+// took 142 us at nside 256, 7 maps, every matrix with one level, this 93
+// (map2alm 224 -> 84).
 // ------------------------------------------------------------------------
 template <int NT>
-__global__ void __launch_bounds__(kThr) k_m2a_level(FastParams p) {
-  constexpr int VT = 8 * NT;
-  constexpr int VP = VT + 8;
-  extern __shared__ double qs[];  // (n rounded to 4) x VP
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int g4 = lane >> 2, t4 = lane & 3;
-  for (int unit = blockIdx.x; unit < p.nroots; unit += gridDim.x) {
-    const DevRootUnit U = p.roots[unit];
+__global__ void __launch_bounds__(kThr) k_a2m_level(FastParams p, int npass) {
+  constexpr int NV = 8 * NT, VP = kLevelPitch<NT>;
+  extern __shared__ double level_smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g4 = lane >> 2, t4 = lane & 3;
+  double *xs = level_smem, *ys = level_smem + p.max_root_k * VP;
+  for (int unit = blockIdx.x; unit < p.nroots * npass; unit += gridDim.x) {
+    const DevRootUnit U = p.roots[unit / npass];
+    const int v0 = (unit % npass) * NV, vn = min(NV, p.nvecs - v0);
     const DevMatrix M = p.mats[U.matrix];
     const DevPair P = p.pairs[U.pair];
-    const int n4 = (P.n + 3) & ~3;
-    const double *qm = p.q_in + (int64_t)(2 * M.m + M.odd) * p.q_mstride;
-    double *X = p.xbuf + M.xrow * p.nvecs;
-    const int mtT = (P.kT + 7) / 8, mtB = (P.kB + 7) / 8, mtiles = mtT + mtB;
-    for (int v0 = 0; v0 < p.nvecs; v0 += VT) {
-      const int vn = min(VT, p.nvecs - v0);
-      __syncthreads();
-      for (int idx = threadIdx.x; idx < n4 * VT; idx += kThr) {
-        const int z = idx / VT, v = idx % VT;
-        double val = 0.0;
-        if (z < P.n && v < vn) val = qm[(int64_t)(P.out_left + z) * p.q_rstride + v0 + v];
-        qs[z * VP + v] = val;
-      }
-      __syncthreads();
-      for (int mt = warp; mt < mtiles; mt += kThr / 32) {
-        const bool isB = mt >= mtT;
-        const int k = isB ? P.kB : P.kT;
-        const int s = (isB ? mt - mtT : mt) * 8 + g4;
-        const int32_t *map = p.i32 + (isB ? P.mapB : P.mapT);
-        const double *ipt = p.f64 + (isB ? P.ipB_t : P.ipT_t);
+    const double *X = p.xbuf + M.xrow * p.nvecs + v0;
+    double *q = p.q + (int64_t)(2 * M.m + M.odd) * p.q_mstride + (int64_t)P.out_left * p.q_rstride + v0;
+    for (int e = threadIdx.x; e < (P.kT + P.kB) * NV; e += kThr) {
+      const int s = e / NV, v = e % NV, row = s < P.kT ? P.inT + s : P.inB + (s - P.kT);
+      xs[s * VP + v] = v < vn ? X[(int64_t)row * p.nvecs + v] : 0.0;
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int part = 0; part < 2; ++part) {
+      const int k = part ? P.kB : P.kT, m = P.n - k;
+      const double *xp = xs + (part ? P.kT * VP : 0), *ip = p.f64 + (part ? P.ipB_t : P.ipT_t);
+      const int32_t *perm = p.i32 + (part ? P.permB : P.permT);
+      auto put = [&](int z, int v, double y) {
+        double *at = ys + z * VP + v;
+        *at = part ? *at + y : y;
+      };
+      for (int e = threadIdx.x; e < k * NV; e += kThr) put(perm[e / NV], e % NV, xp[e / NV * VP + e % NV]);
+      for (int mt = warp; 8 * mt < m; mt += kThr / 32) {
         double acc[NT][2];
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt) acc[nt][0] = acc[nt][1] = 0.0;
-        for (int ks = 0; ks < n4 / 4; ++ks) {
-          const int z = 4 * ks + t4;
-          const double a = w_elem(map, ipt, P.n, k, z, s);
-#pragma unroll
-          for (int nt = 0; nt < NT; ++nt) dmma(acc[nt], a, qs[(4 * ks + t4) * VP + 8 * nt + g4]);
-        }
-        if (s < k) {
-          double *dst = X + (int64_t)((isB ? P.inB : P.inT) + s) * p.nvecs + v0;
+        level_tile<NT>(ip, m, m, k, mt, [&](int j) { return xp + j * VP; }, acc);
+        if (8 * mt + g4 < m) {
+          const int z = perm[k + 8 * mt + g4];
 #pragma unroll
           for (int nt = 0; nt < NT; ++nt) {
-            const int v = 8 * nt + 2 * t4;
-            if (v < vn) dst[v] = acc[nt][0];
-            if (v + 1 < vn) dst[v + 1] = acc[nt][1];
+            put(z, 8 * nt + 2 * t4, acc[nt][0]);
+            put(z, 8 * nt + 2 * t4 + 1, acc[nt][1]);
           }
         }
       }
+      __syncthreads();
     }
+    for (int e = threadIdx.x; e < P.n * NV; e += kThr) {
+      const int z = e / NV, v = e % NV;
+      if (v < vn) q[(int64_t)z * p.q_rstride + v] = ys[z * VP + v];
+    }
+    __syncthreads();  // xs and ys are free for the next unit
+  }
+}
+
+// ------------------------------------------------------------------------
+// map2alm level: one unit = one depth-1 root and 8 NT vectors.  X_T[s] is q~
+// at skeleton row s plus the interpolant's column s against the other rows
+// (in storage order, through the permutation); B likewise.
+// ------------------------------------------------------------------------
+template <int NT>
+__global__ void __launch_bounds__(kThr) k_m2a_level(FastParams p, int npass) {
+  constexpr int NV = 8 * NT, VP = kLevelPitch<NT>;
+  extern __shared__ double level_smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g4 = lane >> 2, t4 = lane & 3;
+  double *qs = level_smem;
+  int32_t *sperm = reinterpret_cast<int32_t *>(level_smem + p.max_root_n * VP);  // T, then B
+  for (int unit = blockIdx.x; unit < p.nroots * npass; unit += gridDim.x) {
+    const DevRootUnit U = p.roots[unit / npass];
+    const int v0 = (unit % npass) * NV, vn = min(NV, p.nvecs - v0);
+    const DevMatrix M = p.mats[U.matrix];
+    const DevPair P = p.pairs[U.pair];
+    const double *q = p.q_in + (int64_t)(2 * M.m + M.odd) * p.q_mstride + (int64_t)P.out_left * p.q_rstride + v0;
+    double *X = p.xbuf + M.xrow * p.nvecs + v0;
+    for (int e = threadIdx.x; e < P.n * NV; e += kThr) {
+      const int z = e / NV, v = e % NV;
+      qs[z * VP + v] = v < vn ? q[(int64_t)z * p.q_rstride + v] : 0.0;
+    }
+    for (int z = threadIdx.x; z < P.n; z += kThr) {
+      sperm[z] = p.i32[P.permT + z];
+      sperm[P.n + z] = p.i32[P.permB + z];
+    }
+    __syncthreads();
+    const int mtT = (P.kT + 7) / 8, mtB = (P.kB + 7) / 8;
+    for (int mt = warp; mt < mtT + mtB; mt += kThr / 32) {
+      const bool isB = mt >= mtT;
+      const int k = isB ? P.kB : P.kT, tile = isB ? mt - mtT : mt, s = 8 * tile + g4;
+      const int32_t *perm = sperm + (isB ? P.n : 0);
+      double acc[NT][2];
+      level_tile<NT>(p.f64 + (isB ? P.ipB : P.ipT), k, k, P.n - k, tile,
+                     [&](int j) { return qs + perm[k + j] * VP; }, acc);
+      if (s < k) {
+        double *dst = X + (int64_t)((isB ? P.inB : P.inT) + s) * p.nvecs;
+        const double *skel = qs + perm[s] * VP;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+          const int v = 8 * nt + 2 * t4;
+          if (v < vn) dst[v] = skel[v] + acc[nt][0];
+          if (v + 1 < vn) dst[v + 1] = skel[v + 1] + acc[nt][1];
+        }
+      }
+    }
+    __syncthreads();  // qs is free for the next unit
   }
 }
 
@@ -216,49 +229,37 @@ __global__ void k_seeds(FastParams p) {
 }
 
 template <int NT>
-cudaError_t launch_nt(int which, const FastParams &prm, int grid, size_t smem, cudaStream_t st) {
-  switch (which) {
-    case 1: {
-      cudaError_t e = cudaFuncSetAttribute(k_a2m_level<NT>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-      k_a2m_level<NT><<<grid, kThr, smem, st>>>(prm);
-      break;
-    }
-    case 2: {
-      cudaError_t e = cudaFuncSetAttribute(k_m2a_level<NT>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-      k_m2a_level<NT><<<grid, kThr, smem, st>>>(prm);
-      break;
-    }
+size_t level_smem(bool alm2map, const FastParams &p) {
+  return alm2map ? (size_t)(p.max_root_k + p.max_root_n) * kLevelPitch<NT> * sizeof(double)
+                 : (size_t)p.max_root_n * (kLevelPitch<NT> * sizeof(double) + 2 * sizeof(int32_t));
+}
+
+template <int NT>
+cudaError_t launch_level_nt(bool alm2map, const FastParams &p, int max_ctas, cudaStream_t st) {
+  const size_t smem = level_smem<NT>(alm2map, p);
+  const int npass = (p.nvecs + 8 * NT - 1) / (8 * NT);
+  const int64_t units = (int64_t)p.nroots * npass;
+  const int grid = (int)std::min<int64_t>(units, max_ctas > 0 ? max_ctas : INT_MAX);
+  auto kernel = alm2map ? k_a2m_level<NT> : k_m2a_level<NT>;
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
   }
+  kernel<<<grid, kThr, smem, st>>>(p, npass);
   return cudaGetLastError();
 }
 
 }  // namespace
 
-int fast_vector_tiles(int nvecs) {
-  // N-tiles of 8 vectors per pass: the smallest power of two covering
-  // nvecs, at most 8 (64 vectors per pass)
-  int nt = 1;
-  while (nt < 8 && 8 * nt < nvecs) nt *= 2;
-  return nt;
-}
-
-cudaError_t launch_fast(int which, const FastParams &prm, int grid, cudaStream_t st) {
-  const int NT = fast_vector_tiles(prm.nvecs);
-  const int VP = 8 * NT + 8;
-  size_t smem = 0;
-  if (which == 1) smem = (size_t)((prm.max_root_k + 3) & ~3) * VP * sizeof(double);
-  if (which == 2) smem = (size_t)((prm.max_root_n + 3) & ~3) * VP * sizeof(double);
-  if (which == 1 || which == 2) smem = smem < 16 ? 16 : smem;
-  switch (NT) {
-    case 1: return launch_nt<1>(which, prm, grid, smem, st);
-    case 2: return launch_nt<2>(which, prm, grid, smem, st);
-    case 4: return launch_nt<4>(which, prm, grid, smem, st);
-    default: return launch_nt<8>(which, prm, grid, smem, st);
-  }
+cudaError_t launch_level(bool alm2map, const FastParams &p, int max_ctas, cudaStream_t st) {
+  if (p.nroots <= 0) return cudaSuccess;
+  // up to 32 vectors per pass, as few as cover them, and no more than leave
+  // room for four CTAs per SM (16 maps at nside 256: 32 vectors per alm2map
+  // pass, 82 KB and two CTAs, took 308 us with the residual)
+  constexpr size_t kRoom = 56 * 1024;
+  if (p.nvecs > 16 && level_smem<4>(alm2map, p) <= kRoom) return launch_level_nt<4>(alm2map, p, max_ctas, st);
+  if (p.nvecs > 8 && level_smem<2>(alm2map, p) <= kRoom) return launch_level_nt<2>(alm2map, p, max_ctas, st);
+  return launch_level_nt<1>(alm2map, p, max_ctas, st);
 }
 
 cudaError_t launch_seeds(const FastParams &prm, cudaStream_t st) {
