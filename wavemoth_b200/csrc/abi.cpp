@@ -151,7 +151,7 @@ struct _wavemoth_plan : ImageRefs {
   int8_t *d_planes = nullptr;
   int32_t *d_status = nullptr;
   wm::DevRingTask *d_ring_tasks = nullptr;
-  int32_t ring_ntasks = 0, ring_smem = 0;
+  int32_t ring_ntasks = 0, ring_smem = 0, ring_threads = 0;
   double *d_alm = nullptr, *d_map = nullptr, *d_q = nullptr, *d_scratch = nullptr;
   double *d_ring_weights = nullptr;           // per ring pair (null: unweighted analysis)
   double *d_ring_weights_buf = nullptr;
@@ -225,6 +225,7 @@ struct RingTable {
   int32_t twlen = 4;         // largest power-of-two table length needed
   int32_t max_bluestein = 0;
   int32_t smem = 0;
+  int32_t threads = 0;
   int32_t nphase_hi = 1;
   int64_t max_cta_cplx = 0;  // largest transform buffer of one CTA
 };
@@ -261,6 +262,23 @@ RingTable ring_table(int nside, int nmaps, int mmax, bool one_side = false) {
   T.nphase_hi = mmax / 64 + 1;
   int gmax = 1;
   while (gmax < nmaps && gmax < 8) gmax <<= 1;
+  // longest transform of one map, both hemispheres, and from it the transform
+  // buffer of a CTA: as small as holds it, so that several CTAs per SM hide
+  // one another's global reads and barriers.  Large batches take twice that:
+  // the groups of maps that read a q row together are wider.  Measured,
+  // synthesis + analysis, buffer of 2048 / 4096 / 8192 points (CTAs of 128 /
+  // 256 / 512 threads): nside 256 (2048 points per map), 1 map 52 / 84 / 126
+  // us, 16 maps 370 / 352 / 372, 32 maps 705 / 640 / 681; nside 512 (4096),
+  // 1 map - / 153 / 215 us, 3 maps - / 371 / 389, 16 maps - / 1439 / 1355;
+  // nside 1024 (8192) has no choice.
+  int longest = 1;
+  for (int r = 0; r < 2 * nside; ++r) {
+    const int N = (int)(offs[mid + r + 1] - offs[mid + r]) / 2;
+    int len = 1;
+    while (len < ((N & (N - 1)) ? 2 * N - 1 : N)) len <<= 1;
+    longest = std::max(longest, 2 * len);
+  }
+  const int buffer = std::min(wm::kRingBufferCplx, std::max(2048, nmaps >= 16 ? 2 * longest : longest));
   struct Item { double cost; wm::DevRingTask t; int64_t cplx; };
   std::vector<Item> items;
   for (int r = 0; r < 2 * nside; ++r) {
@@ -294,7 +312,7 @@ RingTable ring_table(int nside, int nmaps, int mmax, bool one_side = false) {
       two = 0;
       G = std::max(1, std::min(gmax, wm::kRingBufferCplx / len));
     } else if (2 * len <= wm::kRingBufferCplx) {
-      G = std::min(gmax, wm::kRingBufferCplx / (2 * len));
+      G = std::min(gmax, std::max(1, buffer / (2 * len)));
     } else {
       two = 0;
     }
@@ -313,6 +331,7 @@ RingTable ring_table(int nside, int nmaps, int mmax, bool one_side = false) {
     need = std::max(need, it.cplx);
   }
   T.smem = T.tasks.empty() ? 0 : wm::ring_cta_smem(need, T.nphase_hi);
+  T.threads = need > 4096 ? 512 : need > 2048 ? 256 : 128;  // 16 points per thread
   return T;
 }
 
@@ -829,6 +848,7 @@ wavemoth_plan make_plan(bool analysis, int Nside, int lmax, int mmax, int nmaps,
     }
     P->ring_ntasks = (int32_t)RT.tasks.size();
     P->ring_smem = RT.smem;
+    P->ring_threads = RT.threads;
     rc = rc ? rc : upload(A, &P->d_ring_tasks, RT.tasks, "ring work list");
   }
   if (img->split) {
@@ -929,6 +949,7 @@ wm::RingParams ring_params(wavemoth_plan P) {
   r.tasks = P->d_ring_tasks;
   r.ntasks = P->ring_ntasks;
   r.smem = P->ring_smem;
+  r.threads = P->ring_threads;
   r.nphase_hi = P->nphase_hi;
   r.phases = P->d_phases;
   return r;
@@ -1494,6 +1515,7 @@ int wavemoth_plan_set_hemisphere_mode(wavemoth_plan plan, int one_side) {
   plan->d_ring_tasks = tasks;
   plan->ring_ntasks = (int32_t)RT.tasks.size();
   plan->ring_smem = RT.smem;
+  plan->ring_threads = RT.threads;
   return 0;
 }
 

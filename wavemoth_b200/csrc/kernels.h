@@ -210,6 +210,7 @@ struct RingParams {
   const DevRingTask *tasks;
   int32_t ntasks;
   int32_t smem;           // bytes
+  int32_t threads;        // per CTA: 128, 256 or 512
   int32_t nphase_hi;      // entries of the coarse phase table (mmax / 64 + 1)
   // per ring pair, kPhaseLo + nphase_hi phase factors (fine then coarse
   // table), computed at plan creation

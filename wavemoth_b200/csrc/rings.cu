@@ -19,7 +19,7 @@
 // length is not a multiple of 4); a pass loads 16 points per butterfly into
 // registers and runs four radix-2 stages there.  The first radix-16 pass of
 // a decimation in frequency leaves 16 independent blocks per lane; each of
-// the CTA's 16 warps owns one and runs the later passes (the earlier ones of
+// the CTA's warps owns some of them and runs the later passes (the earlier ones of
 // a decimation in time) on it alone, with warp barriers in place of CTA
 // barriers:
 //   * N a power of two (every belt ring): synthesis by decimation in
@@ -42,8 +42,12 @@
 // e^{2 pi i k / n} of the Bluestein rings from a per-ring table; all computed
 // at plan creation with sincospi on exact rationals.
 //
-// Work decomposition: one CTA of 512 threads per (ring pair, group of G = 2^lg
-// maps) with a 128 KB transform buffer (8192 complex, 16 points per thread).
+// Work decomposition: one CTA per (ring pair, group of G = 2^lg maps), of 512
+// threads with a 128 KB transform buffer (8192 complex, 16 points per thread)
+// or, where shorter transforms and few maps allow (ring_table in abi.cpp), of
+// 256 or 128 threads with 64 or 32 KB, two or four to an SM: 512 threads are a
+// whole SM's registers, and a CTA alone on its SM waits out every global read
+// and barrier (nside 256, 1 map: 66 us of synthesis, 29 with four CTAs).
 // Both hemispheres of the pair share the CTA when 2 G x N (or 2 G x M) fits
 // the buffer: lanes are (side, map), so synthesis reads every q element once
 // and analysis writes every q~ element once; longer transforms (nside 2048)
@@ -69,8 +73,6 @@ namespace {
 
 constexpr int kRadixLog = 4;           // largest pass radix 2^kRadixLog
 constexpr int kRingThreads = 512;      // 16 points per thread of a kRingBufferCplx buffer
-constexpr int kRingWarps = kRingThreads / 32;
-static_assert(kRingWarps == 16, "warp-local passes give each of 16 warps the blocks of a radix-16 pass");
 constexpr int kPhaseLo = kRingPhaseLo;  // e^{i m phi0} = hi[m / 64] * lo[m % 64]
 
 struct cplx {
@@ -196,9 +198,12 @@ __device__ __forceinline__ void dit_regs(cplx (&x)[R], const cplx (&A)[Log2<R>::
 namespace wm {
 namespace {
 
-// Shared arguments of the passes of one CTA: the twiddle table (2^lgtw
-// entries), the transform length M and the log2 of the lanes.
+// Shared arguments of the passes of one CTA of kWarps warps: the twiddle
+// table (2^lgtw entries), the transform length M and the log2 of the lanes.
+template <int kWarps>
 struct FftCtx {
+  static constexpr int warps = kWarps;
+  static_assert(16 % kWarps == 0, "warp-local passes divide the 16 blocks of a radix-16 pass among the warps");
   const double2 *tw;
   int lgtw;
   int M;
@@ -212,8 +217,8 @@ struct FftCtx {
 // first radix-16 pass of a decimation in frequency (and before the last of
 // a decimation in time), whose blocks nest in those the warp owns, so that
 // warps run these passes without waiting for one another.
-template <int LR, class BodyF>
-__device__ __forceinline__ void for_butterflies(const FftCtx &f, int wl, BodyF body) {
+template <int LR, class Ctx, class BodyF>
+__device__ __forceinline__ void for_butterflies(const Ctx &f, int wl, BodyF body) {
   const int gm = (1 << f.lg) - 1;
   if (wl == 0) {
     const int nbf = (f.M >> LR) << f.lg;
@@ -221,8 +226,8 @@ __device__ __forceinline__ void for_butterflies(const FftCtx &f, int wl, BodyF b
     __syncthreads();
   } else {
     // warp w owns the blocks [w k, (w + 1) k): nblk >= 16 blocks (a power of
-    // two) over the CTA's 16 warps; its lanes run over (block, butterfly)
-    const int k = (f.M >> wl) / kRingWarps, warp = threadIdx.x >> 5;
+    // two) over the CTA's warps; its lanes run over (block, butterfly)
+    const int k = (f.M >> wl) / Ctx::warps, warp = threadIdx.x >> 5;
     const int lp = wl - LR + f.lg;  // log2 of the butterflies of one block, all lanes
     for (int i = threadIdx.x & 31; i < (k << lp); i += 32) {
       const int B = warp * k + (i >> lp), u = i & ((1 << lp) - 1);
@@ -235,8 +240,8 @@ __device__ __forceinline__ void for_butterflies(const FftCtx &f, int wl, BodyF b
 // One in-place pass of radix R over the 2^lg interleaved sequences of length
 // M: butterfly b of lane g takes the points base + i q (q = len / R, len =
 // 2^lglen) of its block, through `load(index, g)` and `store(index, g, value)`.
-template <int R, int SIGN, bool DIF, class LoadF, class StoreF>
-__device__ __forceinline__ void fft_pass(const FftCtx &f, int lglen, int wl, LoadF load, StoreF store) {
+template <int R, int SIGN, bool DIF, class Ctx, class LoadF, class StoreF>
+__device__ __forceinline__ void fft_pass(const Ctx &f, int lglen, int wl, LoadF load, StoreF store) {
   constexpr int LR = Log2<R>::v;
   const int lq = lglen - LR;
   for_butterflies<LR>(f, wl, [&](int b, int g) {
@@ -253,8 +258,8 @@ __device__ __forceinline__ void fft_pass(const FftCtx &f, int lglen, int wl, Loa
   });
 }
 
-template <int SIGN, bool DIF, class LoadF, class StoreF>
-__device__ __forceinline__ void fft_pass_r(const FftCtx &f, int R, int lglen, int wl, LoadF load, StoreF store) {
+template <int SIGN, bool DIF, class Ctx, class LoadF, class StoreF>
+__device__ __forceinline__ void fft_pass_r(const Ctx &f, int R, int lglen, int wl, LoadF load, StoreF store) {
   switch (R) {
     case 2: fft_pass<2, SIGN, DIF>(f, lglen, wl, load, store); break;
     case 4: fft_pass<4, SIGN, DIF>(f, lglen, wl, load, store); break;
@@ -273,8 +278,8 @@ __device__ __forceinline__ void fft_pass_r(const FftCtx &f, int R, int lglen, in
 // filter spectrum (stored in DIF output order; the sign -1 filter is its
 // reflection F'(k) = conj F(-k)), inverse DIT stages.  Block offset 0: every
 // stage twiddle is 1.
-template <int R, class LoadF, class StoreF>
-__device__ __forceinline__ void bluestein_mid_r(const FftCtx &f, const cplx *F, int fsign, int wl, LoadF load,
+template <int R, class Ctx, class LoadF, class StoreF>
+__device__ __forceinline__ void bluestein_mid_r(const Ctx &f, const cplx *F, int fsign, int wl, LoadF load,
                                                 StoreF store) {
   const int bitsM = ilog2(f.M);
   cplx one[Log2<R>::v];
@@ -305,8 +310,8 @@ __device__ __forceinline__ void bluestein_mid_r(const FftCtx &f, const cplx *F, 
   });
 }
 
-template <class LoadF, class StoreF>
-__device__ __forceinline__ void bluestein_mid(const FftCtx &f, int R, const cplx *F, int fsign, int wl, LoadF load,
+template <class Ctx, class LoadF, class StoreF>
+__device__ __forceinline__ void bluestein_mid(const Ctx &f, int R, const cplx *F, int fsign, int wl, LoadF load,
                                               StoreF store) {
   switch (R) {
     case 2: bluestein_mid_r<2>(f, F, fsign, wl, load, store); break;
@@ -482,7 +487,8 @@ __device__ __forceinline__ void alias_sums(const double *qg, int j, int n, int m
   }
 }
 
-__global__ void __launch_bounds__(kRingThreads, 1) k_ring_synthesis(RingParams p) {
+template <int kThr>
+__global__ void __launch_bounds__(kThr, kRingThreads / kThr) k_ring_synthesis(RingParams p) {
   extern __shared__ double smem_d[];
   const RingCta c = ring_cta(p, blockIdx.x);
   const int lg = c.lg, gm = (1 << lg) - 1, n = c.n, N = c.N, M = c.M;
@@ -497,7 +503,7 @@ __global__ void __launch_bounds__(kRingThreads, 1) k_ring_synthesis(RingParams p
   // the aliasing sums stop at the ring's m limit (null: every m)
   const int mlim = p.ring_mend ? p.ring_mend[c.ring] - 1 : p.mmax;
   const auto rs = radices<false>(M);
-  const FftCtx fx{p.twiddles, ilog2(p.twlen), M, lg};
+  const FftCtx<kThr / 32> fx{p.twiddles, ilog2(p.twlen), M, lg};
   const cplx *F = reinterpret_cast<const cplx *>(p.filters) + c.R.filter;
   const double inv = (c.pow2 ? 1.0 : 1.0 / (double)M) * p.map_scale;
   const int gmm = (1 << c.lgm) - 1;
@@ -604,7 +610,8 @@ __global__ void __launch_bounds__(kRingThreads, 1) k_ring_synthesis(RingParams p
   }
 }
 
-__global__ void __launch_bounds__(kRingThreads, 1) k_ring_analysis(RingParams p) {
+template <int kThr>
+__global__ void __launch_bounds__(kThr, kRingThreads / kThr) k_ring_analysis(RingParams p) {
   extern __shared__ double smem_d[];
   const RingCta c = ring_cta(p, blockIdx.x);
   const int lg = c.lg, n = c.n, N = c.N, M = c.M;
@@ -615,7 +622,7 @@ __global__ void __launch_bounds__(kRingThreads, 1) k_ring_analysis(RingParams p)
   const int64_t half = p.nvecs, qstride = 2 * half;
   double *qbase = p.q_out + (int64_t)c.ring * (p.mmax + 1) * qstride + 2 * c.map0;
   const auto rs = radices<false>(M);
-  const FftCtx fx{p.twiddles, ilog2(p.twlen), M, lg};
+  const FftCtx<kThr / 32> fx{p.twiddles, ilog2(p.twlen), M, lg};
   const cplx *F = reinterpret_cast<const cplx *>(p.filters) + c.R.filter;
   const double inv = c.pow2 ? 1.0 : 1.0 / (double)M;
   const int gmm = (1 << c.lgm) - 1;
@@ -772,7 +779,7 @@ __global__ void __launch_bounds__(kRingThreads) k_bluestein_filters(RingParams p
   auto sload = [&](int i, int g) -> cplx { return buf[at(i, g, 0)]; };
   auto sstore = [&](int i, int g, cplx v) { buf[at(i, g, 0)] = v; };
   const auto rs = radices<true>(M);
-  const FftCtx fx{p.twiddles, ilog2(p.twlen), M, 0};
+  const FftCtx<kRingThreads / 32> fx{p.twiddles, ilog2(p.twlen), M, 0};
   for (int ps = 0; ps < rs.n; ++ps)
     fft_pass_r<-1, true>(fx, rs.r(ps), rs.lgl(ps), 0, sload, sstore);
   cplx *F = reinterpret_cast<cplx *>(p.filters_out) + R.filter;
@@ -780,11 +787,11 @@ __global__ void __launch_bounds__(kRingThreads) k_bluestein_filters(RingParams p
 }
 
 template <class K>
-cudaError_t launch_rings(K kernel, const RingParams &prm, cudaStream_t st) {
+cudaError_t launch_rings(K kernel, int threads, const RingParams &prm, cudaStream_t st) {
   if (prm.ntasks <= 0) return cudaSuccess;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, prm.smem);
   if (e != cudaSuccess) return e;
-  kernel<<<prm.ntasks, kRingThreads, prm.smem, st>>>(prm);
+  kernel<<<prm.ntasks, threads, prm.smem, st>>>(prm);
   return cudaGetLastError();
 }
 
@@ -795,11 +802,19 @@ int32_t ring_cta_smem(int64_t buffer_cplx, int32_t nphase_hi) {
 }
 
 cudaError_t launch_ring_synthesis(const RingParams &prm, cudaStream_t st) {
-  return launch_rings(k_ring_synthesis, prm, st);
+  switch (prm.threads) {
+    case 128: return launch_rings(k_ring_synthesis<128>, 128, prm, st);
+    case 256: return launch_rings(k_ring_synthesis<256>, 256, prm, st);
+    default: return launch_rings(k_ring_synthesis<kRingThreads>, kRingThreads, prm, st);
+  }
 }
 
 cudaError_t launch_ring_analysis(const RingParams &prm, cudaStream_t st) {
-  return launch_rings(k_ring_analysis, prm, st);
+  switch (prm.threads) {
+    case 128: return launch_rings(k_ring_analysis<128>, 128, prm, st);
+    case 256: return launch_rings(k_ring_analysis<256>, 256, prm, st);
+    default: return launch_rings(k_ring_analysis<kRingThreads>, kRingThreads, prm, st);
+  }
 }
 
 __global__ void k_residual(const double *__restrict__ a, const double *__restrict__ b, double *__restrict__ y,
