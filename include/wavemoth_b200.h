@@ -21,7 +21,9 @@ extern "C" {
 #define WAVEMOTH_DEVICE_POINTERS 0x100   /* input/output given at plan time are device pointers */
 #define WAVEMOTH_PRECISION_SPLIT 0x200   /* residual products of depth-0/1 matrices as sliced int8
                                             tensor-core GEMMs re-summed in FP64 (Ozaki scheme);
-                                            the recurrence, seeds and scales stay FP64 */
+                                            the recurrence, seeds and scales stay FP64.  Large
+                                            plans of few maps (up to 8, 14 below nside 512), for
+                                            which that is slower, compute in FP64 throughout */
 #define WAVEMOTH_DENSE 0x800            /* no butterfly file: every (m, parity) block as one dense
                                            three-term recurrence over all rings, seeded on the device
                                            (the reference GPU kernel's scheme, wavemoth/cuda/sht.py:20-148);
@@ -89,7 +91,9 @@ int wavemoth_execute_map2alm_device(wavemoth_plan plan, const double *map, doubl
    device pointers, no ring weights) run as one transform of their summed
    map count, on a plan and interleaved buffers the batch allocates here and
    frees with it; the graph gathers their inputs and scatters the results,
-   which equal those of the separate calls.  Creation must not run inside
+   which equal those of the separate calls (to the split precision where
+   split-precision requests of few maps add up to enough for the split
+   GEMMs).  Creation must not run inside
    another stream capture. */
 typedef struct _wavemoth_batch *wavemoth_batch;
 wavemoth_batch wavemoth_batch_create(int nreq, const wavemoth_plan *plans, const int *directions,
@@ -242,7 +246,8 @@ int wavemoth_plan_set_grid_cap(wavemoth_plan plan, int sms);
    WAVEMOTH_ERR_DEVICE; the kernel then
    waits for the copies and MMAs it already issued, frees its tensor memory
    and returns, so the context stays usable.  With a tiny limit a call
-   fails this way on purpose.  New; it replaces the reference's abort() on a
+   fails this way on purpose.  A plan with a limit set runs these GEMMs
+   also where its few maps would be computed in FP64.  New; it replaces the reference's abort() on a
    failed check (src/wavemoth_error.h:1-19). */
 int wavemoth_plan_set_wait_limit(wavemoth_plan plan, int64_t polls);
 

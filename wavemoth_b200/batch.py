@@ -11,7 +11,10 @@ branches; `execute()` is then one graph launch on torch's current stream.
 Requests of one direction whose Transforms share a device image (same
 plan file, lmax and precision) run as one transform of their summed maps:
 the matrices are streamed once for all of them (`transforms()` counts what
-the graph runs; the results equal the separate calls').
+the graph runs; the results equal the separate calls', bit for bit unless
+split-precision requests of few maps, which run on the FP64 units by
+themselves, add up to enough for the split GEMMs -- then within the split
+precision).
 
 Schedule autotuning: a schedule is the number of branches and, with more
 than one, the SMs each request's persistent Legendre kernels may occupy

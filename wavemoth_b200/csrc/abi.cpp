@@ -441,6 +441,48 @@ struct ImageKey {
 std::mutex g_image_mutex;
 std::map<ImageKey, std::weak_ptr<DeviceImage>> g_images;
 
+// Tables of the FP64 residual path (filled by init_image).
+int build_direct(DeviceImage &I) {
+  auto &G = I.prog;
+  DeviceArena &A = I.arena;
+  const size_t nc = G.gcols.size();
+  int rc = 0;
+  for (int w = 0; w < 2; ++w) {
+    wm::DevDirectTileA *tiles = nullptr;
+    rc = rc ? rc : upload(A, &tiles, G.direct_a[w], "alm2map tiles");
+    I.d_direct_a[w] = tiles;
+    I.ndirect_a[w] = (int32_t)G.direct_a[w].size();
+  }
+  rc = rc ? rc : upload(A, &I.d_direct_b, G.direct_b, "map2alm tiles");
+  I.ndirect_b = (int32_t)G.direct_b.size();
+  rc = rc ? rc : upload(A, &I.d_direct_tile_seeds, G.direct_tile_seeds, "seed tables");
+  rc = rc ? rc : upload(A, &I.d_direct_ab, G.direct_ab, "row coefficients");
+  rc = rc ? rc : upload(A, &I.d_direct_scale, G.direct_scale, "row scales");
+  rc = rc ? rc : A.alloc(&I.d_direct_cols, nc, "column table");
+  rc = rc ? rc : A.alloc(&I.d_direct_inj, nc * wm::kDirectInj, "column first values");
+  rc = rc ? rc : A.alloc(&I.d_direct_seeds, (size_t)G.direct_seeds, "segment seeds");
+  I.direct = rc == 0;
+  return rc;
+}
+
+// The FP64 path of a split image, for its plans of few maps (use_direct):
+// where the plan is large enough to use it, and its tables (at most 8 GiB: an
+// nside 1024 plan's are 5) fit beside everything already on the device with a
+// margin of 4 GiB (and under a memory cap).
+constexpr int64_t kDirectMinElems = 4 << 20;
+
+void build_direct_for_split(DeviceImage &I, int64_t plan_bytes) {
+  const auto &G = I.prog;
+  if (!I.split || G.rec_elems < kDirectMinElems) return;
+  const int64_t need = G.direct_seeds * (int64_t)sizeof(double2) +
+                       (int64_t)G.gcols.size() * (int64_t)(sizeof(wm::DevDirectCol) + wm::kDirectInj * sizeof(double)) +
+                       (int64_t)(G.direct_ab.size() + G.direct_scale.size()) * (int64_t)sizeof(double) + (64LL << 20);
+  size_t fr = 0, tot = 0;
+  if (need > (8LL << 30) || cudaMemGetInfo(&fr, &tot) != cudaSuccess || (int64_t)fr < need + (4LL << 30)) return;
+  if (g_device_cap > 0 && I.arena.bytes + plan_bytes + need > g_device_cap) return;
+  build_direct(I);
+}
+
 // Uploads the map-count independent tables of `img` (whose program is
 // compiled) and allocates its plan-time outputs; the plan-time kernels run
 // later, through the first plan.
@@ -476,24 +518,7 @@ int build_image(DeviceImage &I, int nside, int mmax, unsigned flags) {
   rc = rc ? rc : upload(A, &I.d_gcols, G.gcols, "group columns");
   rc = rc ? rc : upload(A, &I.d_roots, G.roots, "roots");
   I.split = (flags & WAVEMOTH_PRECISION_SPLIT) != 0;
-  I.direct = !I.split;
-  if (I.direct) {
-    const size_t nc = G.gcols.size();
-    for (int w = 0; w < 2; ++w) {
-      wm::DevDirectTileA *tiles = nullptr;
-      rc = rc ? rc : upload(A, &tiles, G.direct_a[w], "alm2map tiles");
-      I.d_direct_a[w] = tiles;
-      I.ndirect_a[w] = (int32_t)G.direct_a[w].size();
-    }
-    rc = rc ? rc : upload(A, &I.d_direct_b, G.direct_b, "map2alm tiles");
-    I.ndirect_b = (int32_t)G.direct_b.size();
-    rc = rc ? rc : upload(A, &I.d_direct_tile_seeds, G.direct_tile_seeds, "seed tables");
-    rc = rc ? rc : upload(A, &I.d_direct_ab, G.direct_ab, "row coefficients");
-    rc = rc ? rc : upload(A, &I.d_direct_scale, G.direct_scale, "row scales");
-    rc = rc ? rc : A.alloc(&I.d_direct_cols, nc, "column table");
-    rc = rc ? rc : A.alloc(&I.d_direct_inj, nc * wm::kDirectInj, "column first values");
-    rc = rc ? rc : A.alloc(&I.d_direct_seeds, (size_t)G.direct_seeds, "segment seeds");
-  }
+  if (!I.split) rc = rc ? rc : build_direct(I);
   if (I.split) rc = rc ? rc : A.alloc(&I.d_seeds, (size_t)std::max<int64_t>(G.nseeds, 1), "recurrence seeds");
   I.program_bytes = A.bytes;
   {
@@ -868,6 +893,7 @@ wavemoth_plan make_plan(bool analysis, int Nside, int lmax, int mmax, int nmaps,
   }
   if (!rc && fresh) {
     alloc_residual_slices(*img, A.bytes, flags);
+    build_direct_for_split(*img, A.bytes);
     A.base = img->arena.bytes;
   }
   static_cast<ImageRefs &>(*P) = static_cast<const ImageRefs &>(*img);
@@ -1053,6 +1079,22 @@ int run_split(wavemoth_plan P, bool alm2map, const double *alm_in, double *alm_o
   return 0;
 }
 
+// Whether a plan's Legendre step runs on the FP64 units: always without split
+// precision, and with it where that is faster.  The split GEMMs stream six
+// bytes of sliced P per element whatever the number of maps, the FP64 kernels
+// do two operations and one per vector.  Measured, alm2map + map2alm, FP64 /
+// split, us: nside 128, lmax 256: 3 maps 43 / 130, 16 maps 106 / 138; nside
+// 256, lmax 512: 8 maps 284 / 485, 16 maps 500 / 507; nside 512, lmax 1024:
+// 8 maps 1501 / 2261, 16 maps 2861 / 2330; nside 1024, lmax 1500: 3 maps 2841
+// / 7254, 8 maps 5474 / 7532, 16 maps 10660 / 7838.  A plan with a wait limit
+// set keeps the kernels whose waits it bounds.
+bool use_direct(wavemoth_plan P) {
+  if (!P->split) return true;
+  if (!P->direct || P->wait_limit > 0) return false;
+  const auto &G = P->img->prog;
+  return P->nvecs <= (G.rec_elems + G.interp_elems <= 80000000 ? 28 : 16);
+}
+
 // FP64 path: residual products, and the interpolation levels of depth-1
 // matrices after (alm2map) or before them (map2alm).
 int run_direct(wavemoth_plan P, bool alm2map, const double *alm_in, double *alm_out, const double *q_in,
@@ -1092,7 +1134,7 @@ int run_legendre(wavemoth_plan P, bool alm2map, const double *alm_in, double *al
   const auto &G = P->img->prog;
   int sp = span_begin(P, alm2map ? 0 : 1, st);
   int rc = 0;
-  if (P->split) {
+  if (!use_direct(P)) {
     rc = run_split(P, alm2map, alm_in, alm_out, q_in, q_out, st);
   } else {
     rc = run_direct(P, alm2map, alm_in, alm_out, q_in, q_out, st);

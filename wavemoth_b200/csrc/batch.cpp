@@ -20,7 +20,9 @@
 // interleaved input and output buffers; inside the graph a copy kernel
 // gathers the requests' inputs before it and scatters the outputs after it.
 // Every map's arithmetic is independent of the other maps', so the results
-// are those of the separate calls.
+// are those of the separate calls (split-precision requests of few maps,
+// whose Legendre step runs on the FP64 units, may add up to enough maps for
+// the split GEMMs: then they agree to the split precision).
 //
 // The plans' own buffers (q, X, operand slices) are shared by all calls on
 // one plan, so a batch must not hold two requests on the same plan.
