@@ -160,7 +160,8 @@ __device__ __forceinline__ void stage_twiddles(cplx (&A)[Log2<R>::v], int j, int
 
 // Radix-R decimation-in-frequency butterfly of R points in registers:
 // log2 R radix-2 stages, stage s multiplied by A[s] and a 16th root.
-template <int R, int SIGN>
+// kHalf: the second half of the points is zero (and not read).
+template <int R, int SIGN, bool kHalf = false>
 __device__ __forceinline__ void dif_regs(cplx (&x)[R], const cplx (&A)[Log2<R>::v]) {
 #pragma unroll
   for (int s = 0; s < Log2<R>::v; ++s) {
@@ -168,6 +169,10 @@ __device__ __forceinline__ void dif_regs(cplx (&x)[R], const cplx (&A)[Log2<R>::
 #pragma unroll
     for (int i = 0; i < R / 2; ++i) {
       const int lo = (i / h) * 2 * h + (i % h), hi = lo + h, m = i % h;
+      if (kHalf && s == 0) {
+        x[hi] = mul_root16<SIGN>(cmul(x[lo], A[0]), m * (16 / R));
+        continue;
+      }
       const cplx u = x[lo], v = x[hi];
       x[lo] = cadd(u, v);
       x[hi] = mul_root16<SIGN>(cmul(csub(u, v), A[s]), (m << s) * (16 / R));
@@ -175,8 +180,9 @@ __device__ __forceinline__ void dif_regs(cplx (&x)[R], const cplx (&A)[Log2<R>::
   }
 }
 
-// Radix-R decimation-in-time butterfly of R points in registers.
-template <int R, int SIGN>
+// Radix-R decimation-in-time butterfly of R points in registers.  kHalf: the
+// second half of the results is not wanted.
+template <int R, int SIGN, bool kHalf = false>
 __device__ __forceinline__ void dit_regs(cplx (&x)[R], const cplx (&A)[Log2<R>::v]) {
 #pragma unroll
   for (int s = 0; s < Log2<R>::v; ++s) {
@@ -187,7 +193,7 @@ __device__ __forceinline__ void dit_regs(cplx (&x)[R], const cplx (&A)[Log2<R>::
       const cplx u = x[lo];
       const cplx t = mul_root16<SIGN>(cmul(x[hi], A[s]), m << (4 - (s + 1)));
       x[lo] = cadd(u, t);
-      x[hi] = csub(u, t);
+      if (!(kHalf && s == Log2<R>::v - 1)) x[hi] = csub(u, t);
     }
   }
 }
@@ -240,7 +246,9 @@ __device__ __forceinline__ void for_butterflies(const Ctx &f, int wl, BodyF body
 // One in-place pass of radix R over the 2^lg interleaved sequences of length
 // M: butterfly b of lane g takes the points base + i q (q = len / R, len =
 // 2^lglen) of its block, through `load(index, g)` and `store(index, g, value)`.
-template <int R, int SIGN, bool DIF, class Ctx, class LoadF, class StoreF>
+// kHalf: a whole-sequence pass whose second half of the sequence is zero
+// before it (DIF) or not wanted after it (DIT).
+template <int R, int SIGN, bool DIF, bool kHalf, class Ctx, class LoadF, class StoreF>
 __device__ __forceinline__ void fft_pass(const Ctx &f, int lglen, int wl, LoadF load, StoreF store) {
   constexpr int LR = Log2<R>::v;
   const int lq = lglen - LR;
@@ -250,27 +258,37 @@ __device__ __forceinline__ void fft_pass(const Ctx &f, int lglen, int wl, LoadF 
     stage_twiddles<R, SIGN, DIF>(A, j, lglen, f.tw, f.lgtw);
     cplx x[R];
 #pragma unroll
-    for (int i = 0; i < R; ++i) x[i] = load(base + (i << lq), g);
-    if (DIF) dif_regs<R, SIGN>(x, A);
-    else dit_regs<R, SIGN>(x, A);
+    for (int i = 0; i < (DIF && kHalf ? R / 2 : R); ++i) x[i] = load(base + (i << lq), g);
+    if (DIF) dif_regs<R, SIGN, kHalf>(x, A);
+    else dit_regs<R, SIGN, kHalf>(x, A);
 #pragma unroll
-    for (int i = 0; i < R; ++i) store(base + (i << lq), g, x[i]);
+    for (int i = 0; i < (!DIF && kHalf ? R / 2 : R); ++i) store(base + (i << lq), g, x[i]);
   });
 }
 
 template <int SIGN, bool DIF, class Ctx, class LoadF, class StoreF>
 __device__ __forceinline__ void fft_pass_r(const Ctx &f, int R, int lglen, int wl, LoadF load, StoreF store) {
   switch (R) {
-    case 2: fft_pass<2, SIGN, DIF>(f, lglen, wl, load, store); break;
-    case 4: fft_pass<4, SIGN, DIF>(f, lglen, wl, load, store); break;
+    case 2: fft_pass<2, SIGN, DIF, false>(f, lglen, wl, load, store); break;
+    case 4: fft_pass<4, SIGN, DIF, false>(f, lglen, wl, load, store); break;
     case 8:
       if (kRadixLog > 3) {
-        fft_pass<8, SIGN, DIF>(f, lglen, wl, load, store);
+        fft_pass<8, SIGN, DIF, false>(f, lglen, wl, load, store);
         break;
       }
       [[fallthrough]];
-    default: fft_pass<(1 << kRadixLog), SIGN, DIF>(f, lglen, wl, load, store); break;
+    default: fft_pass<(1 << kRadixLog), SIGN, DIF, false>(f, lglen, wl, load, store); break;
   }
+}
+
+// The first pass of Bluestein's forward transform (the input is zero from N
+// <= M / 2 on) and the last of its inverse (only the first N results are
+// wanted): radix 16 over the whole sequence, as the first of several DIF
+// passes always is, with half of the reads or writes and of one stage left
+// out.
+template <int SIGN, bool DIF, class Ctx, class LoadF, class StoreF>
+__device__ __forceinline__ void bluestein_end(const Ctx &f, int lglen, LoadF load, StoreF store) {
+  fft_pass<(1 << kRadixLog), SIGN, DIF, true>(f, lglen, 0, load, store);
 }
 
 // Middle of Bluestein's convolution on blocks of R points (R = the last DIF
@@ -491,7 +509,7 @@ template <int kThr>
 __global__ void __launch_bounds__(kThr, kRingThreads / kThr) k_ring_synthesis(RingParams p) {
   extern __shared__ double smem_d[];
   const RingCta c = ring_cta(p, blockIdx.x);
-  const int lg = c.lg, gm = (1 << lg) - 1, n = c.n, N = c.N, M = c.M;
+  const int lg = c.lg, n = c.n, N = c.N, M = c.M;
   cplx *buf = reinterpret_cast<cplx *>(smem_d);
   cplx *plo = buf + ((int64_t)M << lg);
   cplx *phi = plo + kPhaseLo;
@@ -562,11 +580,9 @@ __global__ void __launch_bounds__(kThr, kRingThreads / kThr) k_ring_synthesis(Ri
       qb[0] = nb[0];
       qb[1] = nb[1];
     }
-    if (!c.pow2)
-      for (int t = threadIdx.x; t < ((M - N) << lg); t += blockDim.x)
-        buf[at(N + (t >> lg), t & gm, lg)] = {0.0, 0.0};
     __syncthreads();
     auto sload = [&](int i, int g) -> cplx { return buf[at(i, g, lg)]; };
+    auto zload = [&](int i, int g) -> cplx { return i < N ? buf[at(i, g, lg)] : cplx{0.0, 0.0}; };
     auto sstore = [&](int i, int g, cplx v) { buf[at(i, g, lg)] = v; };
     auto out_row = [&](int g, int64_t pix) -> double * {
       const int64_t off = lane_side(c, g, side) ? c.R.off_south : c.R.off_north;
@@ -592,16 +608,18 @@ __global__ void __launch_bounds__(kThr, kRingThreads / kThr) k_ring_synthesis(Ri
         else fft_pass_r<1, true>(fx, rs.r(ps), rs.lgl(ps), rs.wl(ps), sload, sstore);
       }
     } else {
-      for (int ps = 0; ps < rs.n - 1; ++ps)
-        fft_pass_r<-1, true>(fx, rs.r(ps), rs.lgl(ps), rs.wl(ps), sload, sstore);
+      for (int ps = 0; ps < rs.n - 1; ++ps) {
+        if (ps == 0) bluestein_end<-1, true>(fx, rs.lgl(0), zload, sstore);
+        else fft_pass_r<-1, true>(fx, rs.r(ps), rs.lgl(ps), rs.wl(ps), sload, sstore);
+      }
       const int R = rs.r(rs.n - 1);
       if (rs.n == 1) {
-        bluestein_mid(fx, R, F, +1, 0, sload, pix_blue);
+        bluestein_mid(fx, R, F, +1, 0, zload, pix_blue);
       } else {
         bluestein_mid(fx, R, F, +1, rs.wl(rs.n - 1), sload, sstore);
         for (int ps = rs.n - 2; ps >= 0; --ps) {
           if (rs.wl(ps) == 0 && rs.wl(ps + 1) != 0) __syncthreads();
-          if (ps == 0) fft_pass_r<1, false>(fx, rs.r(ps), rs.lgl(ps), 0, sload, pix_blue);
+          if (ps == 0) bluestein_end<1, false>(fx, rs.lgl(0), sload, pix_blue);
           else fft_pass_r<1, false>(fx, rs.r(ps), rs.lgl(ps), rs.wl(ps), sload, sstore);
         }
       }
@@ -662,7 +680,7 @@ __global__ void __launch_bounds__(kThr, kRingThreads / kThr) k_ring_analysis(Rin
       }
     } else {
       for (int ps = 0; ps < rs.n - 1; ++ps) {
-        if (ps == 0) fft_pass_r<-1, true>(fx, rs.r(ps), rs.lgl(ps), 0, pix_blue, sstore);
+        if (ps == 0) bluestein_end<-1, true>(fx, rs.lgl(0), pix_blue, sstore);
         else fft_pass_r<-1, true>(fx, rs.r(ps), rs.lgl(ps), rs.wl(ps), sload, sstore);
       }
       const int R = rs.r(rs.n - 1);
@@ -672,7 +690,7 @@ __global__ void __launch_bounds__(kThr, kRingThreads / kThr) k_ring_analysis(Rin
         bluestein_mid(fx, R, F, -1, rs.wl(rs.n - 1), sload, sstore);
         for (int ps = rs.n - 2; ps >= 0; --ps) {
           if (rs.wl(ps) == 0 && rs.wl(ps + 1) != 0) __syncthreads();
-          if (ps == 0) fft_pass_r<1, false>(fx, rs.r(ps), rs.lgl(ps), 0, sload, zstore);
+          if (ps == 0) bluestein_end<1, false>(fx, rs.lgl(0), sload, zstore);
           else fft_pass_r<1, false>(fx, rs.r(ps), rs.lgl(ps), rs.wl(ps), sload, sstore);
         }
       }
