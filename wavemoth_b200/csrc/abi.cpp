@@ -543,8 +543,8 @@ int build_image(DeviceImage &I, int nside, int mmax, unsigned flags) {
     rc = rc ? rc : upload(A, &I.d_stiles_la, G.stiles_la, "split alm2map level tiles");
     rc = rc ? rc : upload(A, &I.d_stiles_lm, G.stiles_lm, "split map2alm level tiles");
     rc = rc ? rc : A.alloc(&I.d_level_a,
-                           (size_t)std::max<int64_t>(G.split_level_achunks, 1) * wm::kSplitSlices * wm::kSplitM *
-                               wm::kSplitK, "sliced interpolation matrices");
+                           (size_t)std::max<int64_t>(G.split_level_blocks, 1) * wm::kSplitBlock,
+                           "sliced interpolation matrices");
     rc = rc ? rc : A.alloc(&I.d_level_rs, (size_t)std::max<int64_t>(G.split_level_rows, 1),
                            "interpolation row scales");
     for (int k = 0; k < 4; ++k) {
@@ -563,8 +563,8 @@ int build_image(DeviceImage &I, int nside, int mmax, unsigned flags) {
 // already on the device with a margin of 4 GiB (and under a memory cap).
 void alloc_residual_slices(DeviceImage &I, int64_t plan_bytes, unsigned flags) {
   const auto &G = I.prog;
-  if (!I.split || (flags & WAVEMOTH_SPLIT_GENERATE) || G.stream_res_achunks <= 0) return;
-  const int64_t need = G.stream_res_achunks * (int64_t)wm::kSplitSlices * wm::kSplitM * wm::kSplitK;
+  if (!I.split || (flags & WAVEMOTH_SPLIT_GENERATE) || G.stream_res_blocks <= 0) return;
+  const int64_t need = G.stream_res_blocks * (int64_t)wm::kSplitBlock;
   size_t fr = 0, tot = 0;
   bool fits = cudaMemGetInfo(&fr, &tot) == cudaSuccess && (int64_t)fr > need + (4LL << 30);
   if (g_device_cap > 0 && I.arena.bytes + plan_bytes + need > g_device_cap) fits = false;
@@ -1651,7 +1651,7 @@ int wavemoth_plan_work(wavemoth_plan plan, int nmaps, double *out) {
   // step of 32, nine MMAs with N summing to 1664 (six slices, i + j <= 6)
   double ea = 0.0, eb = 0.0, la = 0.0, lb = 0.0;
   for (const auto &T : G.stiles_a) ea += (double)(G.sgroups[T.group].nrchunks - T.kc0);
-  for (const auto &T : G.stiles_b) eb += (double)G.sgroups[T.group].ncchunks;
+  for (const auto &T : G.stiles_b) eb += (double)T.nk;
   for (const auto &T : G.stiles_la) la += (double)G.sroots[T.unit].nsc;
   for (const auto &T : G.stiles_lm) lb += (double)G.sroots[T.unit].nzc;
   const double chunk = (double)wm::kSplitM * wm::kSplitK;

@@ -297,7 +297,7 @@ __device__ void slice_operand(const SplitParams &p, int gi) {
     G = p.groups[gi];
     const DevSplitGroup S = p.sgroups[gi];
     const DevMatrix M = p.mats[G.matrix];
-    K = kMode == 0 ? G.nrows : G.ncols;
+    K = kMode == 0 ? G.nrows : S.nact;
     nch = kMode == 0 ? S.nrchunks : S.ncchunks;
     plane = kMode == 0 ? S.apl : S.xpl;
     sidx = gi;
@@ -506,13 +506,13 @@ __device__ __forceinline__ bool column_segment(const SplitParams &p, const DevGr
 
 // Scaled digits of 16 values, packed as four words per slice (row i in byte
 // i % 4 of word i / 4), stored as one 16-byte row per slice.
-__device__ __forceinline__ void store_zero_slices(unsigned char *dst) {
+__device__ __forceinline__ void store_zero_slices(unsigned char *dst, int slice = kSliceA) {
 #pragma unroll
-  for (int sl = 0; sl < kSplitSlices; ++sl) *reinterpret_cast<uint4 *>(dst + sl * kSliceA) = make_uint4(0, 0, 0, 0);
+  for (int sl = 0; sl < kSplitSlices; ++sl) *reinterpret_cast<uint4 *>(dst + sl * slice) = make_uint4(0, 0, 0, 0);
 }
 
 __device__ __forceinline__ void store_slices(unsigned char *dst, const double (&v)[16], const double *scale,
-                                             int scale_stride) {
+                                             int scale_stride, int slice = kSliceA) {
   uint32_t w[kSplitSlices][4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -524,7 +524,7 @@ __device__ __forceinline__ void store_slices(unsigned char *dst, const double (&
   }
 #pragma unroll
   for (int sl = 0; sl < kSplitSlices; ++sl)
-    *reinterpret_cast<uint4 *>(dst + sl * kSliceA) = make_uint4(w[sl][0], w[sl][1], w[sl][2], w[sl][3]);
+    *reinterpret_cast<uint4 *>(dst + sl * slice) = make_uint4(w[sl][0], w[sl][1], w[sl][2], w[sl][3]);
 }
 
 struct Pipe {
@@ -726,7 +726,7 @@ __global__ void __launch_bounds__(kSplitThr, 1) k_m2a_split(SplitParams p) {
       rsc[tid] = tid < T.nrows ? p.row_scale[S.rowoff + T.row0 + tid] : make_double2(0.0, 0.0);
     __syncthreads();
     const int r0 = T.row0 + 16 * seg;
-    for (int kc = 0; kc < S.ncchunks; ++kc) {
+    for (int kc = 0; kc < T.nk; ++kc) {
       const bool ok = stage_free(ss, q);
       stage_load_b(p, smem, q, S.xpl + kc);
       const int64_t gc = (int64_t)kc * kSplitK + cl;
@@ -806,7 +806,9 @@ __global__ void __launch_bounds__(kSplitM) k_level_slices(SplitParams p) {
   for (int k = 0; k < K; ++k) mx = fmax(mx, fabs(w(k)));
   const double2 sc = operand_scale(mx);
   if (act) p.level_rs[(a2m ? R.rs_a2m : R.rs_m2a) + row] = sc;
-  int8_t *A = p.level_a + ((a2m ? R.a_a2m : R.a_m2a) + (int64_t)(T.row0 / kSplitM) * nk) * (int64_t)kStageA;
+  const int blocks = (T.nrows + 15) / 16, slice = blocks * kSplitBlockRow;
+  if (r >= 16 * blocks) return;
+  int8_t *A = p.level_a + ((a2m ? R.a_a2m : R.a_m2a) + (int64_t)(T.row0 / 16) * nk) * (int64_t)kSplitBlock;
   for (int c = 0; c < nk; ++c) {
     for (int h = 0; h < kSplitK / 16; ++h) {
       double v[16];
@@ -821,10 +823,10 @@ __global__ void __launch_bounds__(kSplitM) k_level_slices(SplitParams p) {
 #pragma unroll
         for (int sl = 0; sl < kSplitSlices; ++sl) wd[sl][j] = pack4(d[0][sl], d[1][sl], d[2][sl], d[3][sl]);
       }
-      int8_t *dst = A + (int64_t)c * kStageA + (r >> 3) * 512 + h * 128 + (r & 7) * 16;
+      int8_t *dst = A + (int64_t)c * kSplitSlices * slice + (r >> 3) * 512 + h * 128 + (r & 7) * 16;
 #pragma unroll
       for (int sl = 0; sl < kSplitSlices; ++sl)
-        *reinterpret_cast<uint4 *>(dst + sl * kSliceA) = make_uint4(wd[sl][0], wd[sl][1], wd[sl][2], wd[sl][3]);
+        *reinterpret_cast<uint4 *>(dst + sl * slice) = make_uint4(wd[sl][0], wd[sl][1], wd[sl][2], wd[sl][3]);
     }
   }
 }
@@ -968,8 +970,16 @@ __global__ void __launch_bounds__(kStreamThr, 1) k_stream_split(SplitParams p, S
           const long long use = g / kStreamStages;
           if (use > 0 && !mbar_wait_or_abort(&ss->empty[s], (uint32_t)((use - 1) & 1), abort, lim)) break;
           const uint32_t dst = smem_u32(smem + s * kStreamStage);
-          expect_tx(&ss->full[s], kStreamStage);
-          bulk_load(dst, L.a + (T.a + c) * (int64_t)kStageA, kStageA, &ss->full[s]);
+          // a group's last tile brings its own rows only; the others' lanes are not stored
+          const uint32_t slice = (uint32_t)T.blocks * kSplitBlockRow;
+          const int8_t *a = L.a + (T.a + (int64_t)c * T.blocks) * kSplitBlock;
+          expect_tx(&ss->full[s], kSplitSlices * slice + kStageB);
+          if (slice == kSliceA) {
+            bulk_load(dst, a, kStageA, &ss->full[s]);
+          } else {
+            for (int sl = 0; sl < kSplitSlices; ++sl)
+              bulk_load(dst + sl * kSliceA, a + sl * slice, slice, &ss->full[s]);
+          }
           bulk_load(dst + kStageA, p.planes + (T.b + c) * (int64_t)kSplitPlane, kStageB, &ss->full[s]);
         }
       }
@@ -1088,12 +1098,15 @@ __global__ void __launch_bounds__(kSplitThr) k_res_slices_a2m(SplitParams p, Str
   } else {
     C.start = G.nrows;
   }
-  unsigned char *A = reinterpret_cast<unsigned char *>(const_cast<int8_t *>(L.a)) + ST.a * (int64_t)kStageA;
+  const int slice = ST.blocks * kSplitBlockRow;
+  if (c >= 16 * ST.blocks) return;
+  unsigned char *A = reinterpret_cast<unsigned char *>(const_cast<int8_t *>(L.a)) + ST.a * (int64_t)kSplitBlock;
   for (int kc = T.kc0; kc < S.nrchunks; ++kc) {
-    unsigned char *dst = A + (int64_t)(kc - T.kc0) * kStageA + (c >> 3) * 512 + seg * 128 + (c & 7) * 16;
+    unsigned char *dst =
+        A + (int64_t)(kc - T.kc0) * kSplitSlices * slice + (c >> 3) * 512 + seg * 128 + (c & 7) * 16;
     double v[16];
-    if (column_segment(p, G, C, gc, kc * kSplitK + 16 * seg, v)) store_slices(dst, v, &csc.x, 0);
-    else store_zero_slices(dst);
+    if (column_segment(p, G, C, gc, kc * kSplitK + 16 * seg, v)) store_slices(dst, v, &csc.x, 0, slice);
+    else store_zero_slices(dst, slice);
   }
 }
 
@@ -1108,16 +1121,18 @@ __global__ void __launch_bounds__(kSplitThr) k_res_slices_m2a(SplitParams p, Str
   if (tid < kSplitM) rsc[tid] = tid < T.nrows ? p.row_scale[S.rowoff + T.row0 + tid] : make_double2(0.0, 0.0);
   __syncthreads();
   const int r0 = T.row0 + 16 * seg;
-  unsigned char *A = reinterpret_cast<unsigned char *>(const_cast<int8_t *>(L.a)) + ST.a * (int64_t)kStageA;
-  for (int kc = 0; kc < S.ncchunks; ++kc) {
+  const int slice = ST.blocks * kSplitBlockRow;
+  if (seg >= ST.blocks) return;
+  unsigned char *A = reinterpret_cast<unsigned char *>(const_cast<int8_t *>(L.a)) + ST.a * (int64_t)kSplitBlock;
+  for (int kc = 0; kc < T.nk; ++kc) {
     const int64_t gc = (int64_t)kc * kSplitK + cl;
     DevGCol C{};
     if (gc < G.ncols) C = p.gcols[G.cols + gc];
     else C.start = G.nrows;
-    unsigned char *dst = A + (int64_t)kc * kStageA + seg * 1024 + (cl >> 3) * 128 + (cl & 7) * 16;
+    unsigned char *dst = A + (int64_t)kc * kSplitSlices * slice + seg * 1024 + (cl >> 3) * 128 + (cl & 7) * 16;
     double v[16];
-    if (column_segment(p, G, C, gc, r0, v)) store_slices(dst, v, &rsc[16 * seg].x, 2);
-    else store_zero_slices(dst);
+    if (column_segment(p, G, C, gc, r0, v)) store_slices(dst, v, &rsc[16 * seg].x, 2, slice);
+    else store_zero_slices(dst, slice);
   }
 }
 

@@ -149,21 +149,27 @@ constexpr int kSplitK = 64;       // K chunk (rows for alm2map, columns for map2
 constexpr int kSplitM = 128;      // M tile (columns for alm2map, rows for map2alm)
 constexpr int kSplitN = 64;       // vectors per pass
 constexpr int kSplitPlane = kSplitSlices * kSplitN * kSplitK;  // bytes of one operand chunk
+// A chunks hold the rows that a tile has, in blocks of 16: per slice
+// `blocks` x kSplitBlockRow bytes, slice after slice
+constexpr int kSplitBlockRow = 16 * kSplitK;
+constexpr int kSplitBlock = kSplitSlices * kSplitBlockRow;
 
 struct DevSplitGroup {
   int64_t apl;        // first alm-operand chunk (alm2map): ceil(nrows / kSplitK) chunks
   int64_t xpl;        // first X-operand chunk (map2alm): ceil(ncols / kSplitK) chunks
   int64_t rowoff;     // first entry of the group's row scales
   int32_t nrchunks;
-  int32_t ncchunks;
+  int32_t ncchunks;   // of the columns that have an active row, a prefix
+  int32_t nact;       // their number
+  int32_t pad;
 };
 
 struct DevSplitTileA {  // alm2map: <= kSplitM columns of a group, K chunks from kc0
   int32_t group, col0, ncols, kc0;
 };
 
-struct DevSplitTileB {  // map2alm: <= kSplitM rows of a group, all its columns
-  int32_t group, row0, nrows, pad;
+struct DevSplitTileB {  // map2alm: <= kSplitM rows of a group; K chunks of the columns that start before its end
+  int32_t group, row0, nrows, nk;
 };
 
 // Split-precision level products of a depth-1 root (T, B) pair, W[z][s] the
@@ -171,9 +177,9 @@ struct DevSplitTileB {  // map2alm: <= kSplitM rows of a group, all its columns
 //   alm2map   q[z] = sum_s W[z][s] X[s]     M = z (n), K = s (kT + kB)
 //   map2alm   X[s] = sum_z W[z][s] q~[z]    M = s,     K = z
 // W is sliced once per plan into A chunks laid out as shared memory wants
-// them (kSplitSlices x kSplitM x kSplitK bytes each), per-row scales.
+// them, per-row scales.
 struct DevSplitRoot {
-  int64_t a_a2m, a_m2a;     // first A chunk of each direction (M tiles x K chunks)
+  int64_t a_a2m, a_m2a;     // first A block of each direction (M tiles x K chunks)
   int64_t b_a2m, b_m2a;     // first operand-B chunk (X over s, q~ over z)
   int64_t rs_a2m, rs_m2a;   // first row scale (n rows, kT + kB rows)
   int32_t nzc, nsc;         // chunks of 64 over z and over s
@@ -204,12 +210,12 @@ struct DevSplitLevelTile {  // <= kSplitM rows (z or s) of one root unit
 // destination buffer (-1: none), scaled by 1 / scale of that tile row
 // (entry scale_idx[tile * kSplitM + r] of the launch's scale table).
 struct DevStreamTile {
-  int64_t a;       // first A chunk (kSplitSlices x kSplitM x kSplitK bytes each)
+  int64_t a;       // first A block; a chunk is `blocks` of them
   int64_t b;       // first B plane (kSplitPlane bytes each)
   int32_t nk;      // K chunks (> 0)
   int32_t vs;      // vector-scale row: group, or ngroups + root unit
   int32_t buf;     // destination: 0 q, 1 X buffer, 2 alm
-  int32_t pad;
+  int32_t blocks;  // 16-row blocks of the tile (kSplitM / 16, fewer in a group's last tile)
 };
 
 // Per ring pair (ring number r from the equator).

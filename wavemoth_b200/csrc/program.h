@@ -45,13 +45,13 @@ struct HostProgram {
   int64_t split_rows = 0;               // row scales (sum of group rows)
   std::vector<DevSplitRoot> sroots;     // one per root unit
   std::vector<DevSplitLevelTile> stiles_la, stiles_lm;  // alm2map / map2alm level tiles
-  int64_t split_level_achunks = 0;      // A chunks of W, both directions
+  int64_t split_level_blocks = 0;       // A blocks of W, both directions
   int64_t split_level_rows = 0;         // row scales of W, both directions
   // streamed split GEMM launches (kStream* order): the tiles, and per tile
   // row its destination row and scale index (-1: padding row)
   std::vector<DevStreamTile> stream_tiles[4];
   std::vector<int32_t> stream_rows[4], stream_sidx[4];
-  int64_t stream_res_achunks = 0;       // A chunks of sliced residual P, both directions
+  int64_t stream_res_blocks = 0;        // A blocks of sliced residual P, both directions
   // destination rows that no split tile writes (columns with no active row,
   // roots with no skeleton) and that must read as zero, per launch
   // (kStream* order); encoded kZeroBufShift-bit buffer (0 q, 1 X, 2 alm)
