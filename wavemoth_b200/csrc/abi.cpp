@@ -1097,8 +1097,9 @@ bool use_direct(wavemoth_plan P) {
 
 // FP64 path: residual products, and the interpolation levels of depth-1
 // matrices after (alm2map) or before them (map2alm).
+// accumulate: map2alm adds to the alm.
 int run_direct(wavemoth_plan P, bool alm2map, const double *alm_in, double *alm_out, const double *q_in,
-               double *q_out, cudaStream_t st) {
+               double *q_out, cudaStream_t st, bool accumulate) {
   const auto &G = P->img->prog;
   const int nr = (int)G.roots.size(), cap = P->grid_cap > 0 ? 4 * plan_sms(P) : 0;
   int rc = 0;
@@ -1115,6 +1116,7 @@ int run_direct(wavemoth_plan P, bool alm2map, const double *alm_in, double *alm_
   d.alm_out = alm_out;
   d.q_in = q_in;
   d.q = q_out;
+  d.accumulate = accumulate;
   if (alm2map) {
     d.aligned = (((uintptr_t)q_out | (uintptr_t)alm_in) & 15) == 0;
     rc = cuda_check(wm::launch_direct_a2m(d, P->d_direct_a, P->ndirect_a, plan_sms(P), cap, st),
@@ -1129,15 +1131,16 @@ int run_direct(wavemoth_plan P, bool alm2map, const double *alm_in, double *alm_
   return rc;
 }
 
+// accumulate (map2alm, where accumulates(P)): adds to the alm.
 int run_legendre(wavemoth_plan P, bool alm2map, const double *alm_in, double *alm_out,
-                 const double *q_in, double *q_out, cudaStream_t st) {
+                 const double *q_in, double *q_out, cudaStream_t st, bool accumulate = false) {
   const auto &G = P->img->prog;
   int sp = span_begin(P, alm2map ? 0 : 1, st);
   int rc = 0;
   if (!use_direct(P)) {
     rc = run_split(P, alm2map, alm_in, alm_out, q_in, q_out, st);
   } else {
-    rc = run_direct(P, alm2map, alm_in, alm_out, q_in, q_out, st);
+    rc = run_direct(P, alm2map, alm_in, alm_out, q_in, q_out, st, accumulate);
   }
   if (!rc && P->nslow > 0) {
     wm::LegendreParams p = legendre_params(P);
@@ -1157,8 +1160,13 @@ int run_legendre(wavemoth_plan P, bool alm2map, const double *alm_in, double *al
   return rc;
 }
 
-// scale multiplies the maps (1 for alm2map; 4 pi / npix for the adjoint of map2alm)
-int run_alm2map(wavemoth_plan P, const double *alm, double *map, cudaStream_t st, double scale = 1.0) {
+// Whether the plan's map2alm can add to the alm: every matrix on the FP64 units.
+bool accumulates(wavemoth_plan P) { return use_direct(P) && P->nslow == 0; }
+
+// scale multiplies the maps (1 for alm2map; 4 pi / npix for the adjoint of
+// map2alm); sub, if given, is what they are subtracted from
+int run_alm2map(wavemoth_plan P, const double *alm, double *map, cudaStream_t st, double scale = 1.0,
+                const double *sub = nullptr) {
   if (int rc = run_legendre(P, true, alm, nullptr, nullptr, P->d_q, st)) return rc;
   wm::RingParams r = ring_params(P);
   r.q = P->d_q;
@@ -1167,6 +1175,7 @@ int run_alm2map(wavemoth_plan P, const double *alm, double *map, cudaStream_t st
   // writer's inclusion threshold), and the gather stops there
   r.ring_mend = P->d_ring_mend;
   r.map = map;
+  r.map_sub = sub;
   r.map_scale = scale;
   int sp = span_begin(P, 2, st);
   int rc = cuda_check(wm::launch_ring_synthesis(r, st), "ring synthesis launch");
@@ -1176,7 +1185,8 @@ int run_alm2map(wavemoth_plan P, const double *alm, double *map, cudaStream_t st
 }
 
 // scale multiplies q~ (4 pi / npix for map2alm; 1 for the adjoint of alm2map)
-int run_map2alm(wavemoth_plan P, const double *map, double *alm, cudaStream_t st, double scale = -1.0) {
+int run_map2alm(wavemoth_plan P, const double *map, double *alm, cudaStream_t st, double scale = -1.0,
+                bool accumulate = false) {
   wm::RingParams r = ring_params(P);
   r.map_in = map;
   r.q_out = P->d_q;
@@ -1189,7 +1199,7 @@ int run_map2alm(wavemoth_plan P, const double *map, double *alm, cudaStream_t st
   P->kernel_launches += r.ntasks > 0;
   span_end(P, sp, st);
   if (rc0) return rc0;
-  return run_legendre(P, false, nullptr, alm, P->d_q, nullptr, st);
+  return run_legendre(P, false, nullptr, alm, P->d_q, nullptr, st, accumulate);
 }
 
 // Reads (and clears) the device status word; the stream must be idle.
@@ -1489,19 +1499,19 @@ int wavemoth_map2alm_iterative_device(wavemoth_plan plan, const double *map, dou
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t nmap = plan->npix * plan->nmaps, nalm = plan->nalm * plan->nvecs;
   int rc = 0;
-  if (niter > 0 && !plan->d_iter_map) {
-    rc = plan->arena.alloc(&plan->d_iter_map, (size_t)nmap, "iteration map buffer");
+  const bool add = accumulates(plan);
+  if (niter > 0 && !plan->d_iter_map) rc = plan->arena.alloc(&plan->d_iter_map, (size_t)nmap, "iteration map buffer");
+  if (niter > 0 && !add && !plan->d_iter_alm)
     rc = rc ? rc : plan->arena.alloc(&plan->d_iter_alm, (size_t)nalm, "iteration alm buffer");
-    if (rc) return finish(plan, rc);
-  }
+  if (rc) return finish(plan, rc);
   rc = run_map2alm(plan, map, alm, st);
   for (int it = 0; it < niter && !rc; ++it) {
     // a += map2alm(f - alm2map(a))
-    rc = run_alm2map(plan, alm, plan->d_iter_map, st);
-    if (!rc) rc = cuda_check(wm::launch_residual(map, plan->d_iter_map, plan->d_iter_map, nmap, st), "residual");
-    if (!rc) rc = run_map2alm(plan, plan->d_iter_map, plan->d_iter_alm, st);
-    if (!rc) rc = cuda_check(wm::launch_accumulate(plan->d_iter_alm, alm, nalm, st), "accumulate");
-    plan->kernel_launches += 2;
+    rc = run_alm2map(plan, alm, plan->d_iter_map, st, 1.0, map);
+    if (!rc) rc = run_map2alm(plan, plan->d_iter_map, add ? alm : plan->d_iter_alm, st, -1.0, add);
+    if (rc || add) continue;
+    rc = cuda_check(wm::launch_accumulate(plan->d_iter_alm, alm, nalm, st), "accumulate");
+    plan->kernel_launches++;
   }
   return finish(plan, rc);
 }

@@ -82,7 +82,8 @@ struct DirectParams {
   double *q;
   int64_t q_mstride, q_rstride;
   double *xbuf;
-  int32_t aligned;              // the alm and q are 16-byte aligned
+  int32_t aligned;              // the alm and q are 16-byte aligned (alm2map)
+  int32_t accumulate;           // map2alm: adds to the alm
 };
 
 // max_ctas > 0 bounds the grid (the units are then walked by fewer CTAs);
@@ -192,6 +193,7 @@ struct RingParams {
   const int32_t *ring_mend;  // per ring pair m limit (null: mmax + 1): synthesis sums m < ring_mend[r],
                              // analysis writes zero q~ rows from there on
   double *map;            // synthesis output (npix, nmaps)
+  const double *map_sub;  // synthesis: writes map_sub - map (null: the map)
   const double *map_in;   // analysis input (npix, nmaps)
   double *q_out;          // analysis output
   double scale;           // analysis: multiplies q~ (4 pi / npix for map2alm)
@@ -224,9 +226,7 @@ cudaError_t launch_strided_copy(double *dst, int64_t dpitch, const double *src, 
                                 int64_t rows, cudaStream_t st);
 
 cudaError_t launch_ring_synthesis(const RingParams &prm, cudaStream_t st);
-// y = a - b (n doubles), and y += x (n doubles): the steps of the iterative
-// map2alm between the transforms
-cudaError_t launch_residual(const double *a, const double *b, double *y, int64_t n, cudaStream_t st);
+// y += x (n doubles).
 cudaError_t launch_accumulate(const double *x, double *y, int64_t n, cudaStream_t st);
 // m-sharded plans: moves the 2 nvecs doubles of every (ring of this part,
 // m) between the ring-side q (row (ring (mmax + 1) + m) 2 + parity, rings

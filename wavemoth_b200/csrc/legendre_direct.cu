@@ -127,7 +127,6 @@ __global__ void __launch_bounds__(kDirectThr, direct_ctas(NV * C)) k_direct_a2m(
         copy8(&to.scale[tid], p.scale + G.coef + r0 + tid, true);
       }
     };
-    if (T.kstart < R) fetch(T.kstart, s_chunk[0]);
     // columns of this thread
     double x2[C], y0[C], y1[C], acc[C][NV];
     int row[C];
@@ -149,6 +148,7 @@ __global__ void __launch_bounds__(kDirectThr, direct_ctas(NV * C)) k_direct_a2m(
 #pragma unroll
       for (int v = 0; v < NV; ++v) acc[j][v] = 0.0;
     }
+    if (T.kstart < R) fetch(T.kstart, s_chunk[0]);
     w0 = __reduce_min_sync(0xffffffffu, w0);
     wf = __reduce_max_sync(0xffffffffu, wf);
     dense = __any_sync(0xffffffffu, dense);
@@ -405,10 +405,12 @@ __global__ void __launch_bounds__(kDirectThr, NT == 2 ? 3 : 4) k_direct_m2a(Dire
         __syncthreads();
         for (int e = tid; e < 8 * nr; e += kDirectThr) {
           const int r = e >> 3, v = e & 7, at = 8 * (r % S) + r / S;
-          if (8 * nt + v < vn)
-            dst[2 * (int64_t)r * p.nvecs + 8 * nt + v] =
-                ((s_red[0][at][v] + s_red[1][at][v]) + (s_red[2][at][v] + s_red[3][at][v])) *
-                p.scale[G.coef + T.row0 + r];
+          if (8 * nt + v < vn) {
+            double *to = dst + 2 * (int64_t)r * p.nvecs + 8 * nt + v;
+            const double a = ((s_red[0][at][v] + s_red[1][at][v]) + (s_red[2][at][v] + s_red[3][at][v])) *
+                             p.scale[G.coef + T.row0 + r];
+            *to = p.accumulate ? *to + a : a;
+          }
         }
       }
     }
@@ -464,9 +466,10 @@ __global__ void k_direct_setup(DirectParams p, const DevGCol *gcols, const doubl
 }  // namespace
 
 template <int NV>
-static void a2m(const DirectParams &p, int width, int npass, int grid, cudaStream_t st) {
+static cudaError_t a2m(const DirectParams &p, int width, int npass, int grid, cudaStream_t st) {
   if (width) k_direct_a2m<NV, 2><<<grid, kDirectThr, 0, st>>>(p, npass);
   else k_direct_a2m<NV, 1><<<grid, kDirectThr, 0, st>>>(p, npass);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_direct_a2m(DirectParams p, const DevDirectTileA *const (&tiles)[2], const int32_t (&ntiles)[2],
@@ -488,14 +491,13 @@ cudaError_t launch_direct_a2m(DirectParams p, const DevDirectTileA *const (&tile
   if (units <= 0) return cudaSuccess;
   const int grid = (int)std::min<int64_t>(units, max_ctas > 0 ? max_ctas : INT_MAX);
   switch (nv) {
-    case 2: a2m<2>(p, width, npass, grid, st); break;
-    case 4: a2m<4>(p, width, npass, grid, st); break;
-    case 6: a2m<6>(p, width, npass, grid, st); break;
-    case 8: a2m<8>(p, width, npass, grid, st); break;
-    case 12: a2m<12>(p, width, npass, grid, st); break;
-    default: a2m<16>(p, width, npass, grid, st); break;
+    case 2: return a2m<2>(p, width, npass, grid, st);
+    case 4: return a2m<4>(p, width, npass, grid, st);
+    case 6: return a2m<6>(p, width, npass, grid, st);
+    case 8: return a2m<8>(p, width, npass, grid, st);
+    case 12: return a2m<12>(p, width, npass, grid, st);
+    default: return a2m<16>(p, width, npass, grid, st);
   }
-  return cudaGetLastError();
 }
 
 cudaError_t launch_direct_m2a(const DirectParams &p, int max_ctas, cudaStream_t st) {

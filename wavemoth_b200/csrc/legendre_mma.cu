@@ -156,13 +156,13 @@ __global__ void __launch_bounds__(kThr) k_m2a_level(FastParams p, int npass) {
     const DevPair P = p.pairs[U.pair];
     const double *q = p.q_in + (int64_t)(2 * M.m + M.odd) * p.q_mstride + (int64_t)P.out_left * p.q_rstride + v0;
     double *X = p.xbuf + M.xrow * p.nvecs + v0;
-    for (int e = threadIdx.x; e < P.n * NV; e += kThr) {
-      const int z = e / NV, v = e % NV;
-      qs[z * VP + v] = v < vn ? q[(int64_t)z * p.q_rstride + v] : 0.0;
-    }
     for (int z = threadIdx.x; z < P.n; z += kThr) {
       sperm[z] = p.i32[P.permT + z];
       sperm[P.n + z] = p.i32[P.permB + z];
+    }
+    for (int e = threadIdx.x; e < P.n * NV; e += kThr) {
+      const int z = e / NV, v = e % NV;
+      qs[z * VP + v] = v < vn ? q[(int64_t)z * p.q_rstride + v] : 0.0;
     }
     __syncthreads();
     const int mtT = (P.kT + 7) / 8, mtB = (P.kB + 7) / 8;

@@ -505,7 +505,8 @@ __device__ __forceinline__ void alias_sums(const double *qg, int j, int n, int m
   }
 }
 
-template <int kThr>
+// kSub: writes map_sub - map instead of the map.
+template <int kThr, bool kSub>
 __global__ void __launch_bounds__(kThr, kRingThreads / kThr) k_ring_synthesis(RingParams p) {
   extern __shared__ double smem_d[];
   const RingCta c = ring_cta(p, blockIdx.x);
@@ -588,19 +589,20 @@ __global__ void __launch_bounds__(kThr, kRingThreads / kThr) k_ring_synthesis(Ri
       const int64_t off = lane_side(c, g, side) ? c.R.off_south : c.R.off_north;
       return p.map + (off + pix) * p.nmaps + c.map0 + lane_map(c, g);
     };
+    auto put = [&](double *pixel, double y) { *pixel = kSub ? p.map_sub[pixel - p.map] - y : y; };
     // pixels 2s, 2s + 1 of output z[s]; power of two: DIF position pos holds z[bitrev(pos)]
     auto pix_dif = [&](int pos, int g, cplx z) {
       if (!lane_live(c, g, side)) return;
       z = cscale(z, p.map_scale);
       const int64_t s2 = 2 * (int64_t)bitrev((unsigned)pos, c.bits);
-      *out_row(g, s2) = z.x;
-      *out_row(g, s2 + 1) = z.y;
+      put(out_row(g, s2), z.x);
+      put(out_row(g, s2 + 1), z.y);
     };
     auto pix_blue = [&](int k, int g, cplx z) {
       if (k >= N || !lane_live(c, g, side)) return;
       z = cscale(cmul(z, ring_chirp(p, c.R, k)), inv);
-      *out_row(g, 2 * (int64_t)k) = z.x;
-      *out_row(g, 2 * (int64_t)k + 1) = z.y;
+      put(out_row(g, 2 * (int64_t)k), z.x);
+      put(out_row(g, 2 * (int64_t)k + 1), z.y);
     };
     if (c.pow2) {
       for (int ps = 0; ps < rs.n; ++ps) {
@@ -807,10 +809,21 @@ __global__ void __launch_bounds__(kRingThreads) k_bluestein_filters(RingParams p
 template <class K>
 cudaError_t launch_rings(K kernel, int threads, const RingParams &prm, cudaStream_t st) {
   if (prm.ntasks <= 0) return cudaSuccess;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, prm.smem);
-  if (e != cudaSuccess) return e;
+  if (prm.smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, prm.smem);
+    if (e != cudaSuccess) return e;
+  }
   kernel<<<prm.ntasks, threads, prm.smem, st>>>(prm);
   return cudaGetLastError();
+}
+
+template <bool kSub>
+cudaError_t launch_synthesis(const RingParams &prm, cudaStream_t st) {
+  switch (prm.threads) {
+    case 128: return launch_rings(k_ring_synthesis<128, kSub>, 128, prm, st);
+    case 256: return launch_rings(k_ring_synthesis<256, kSub>, 256, prm, st);
+    default: return launch_rings(k_ring_synthesis<kRingThreads, kSub>, kRingThreads, prm, st);
+  }
 }
 
 }  // namespace
@@ -820,11 +833,7 @@ int32_t ring_cta_smem(int64_t buffer_cplx, int32_t nphase_hi) {
 }
 
 cudaError_t launch_ring_synthesis(const RingParams &prm, cudaStream_t st) {
-  switch (prm.threads) {
-    case 128: return launch_rings(k_ring_synthesis<128>, 128, prm, st);
-    case 256: return launch_rings(k_ring_synthesis<256>, 256, prm, st);
-    default: return launch_rings(k_ring_synthesis<kRingThreads>, kRingThreads, prm, st);
-  }
+  return prm.map_sub ? launch_synthesis<true>(prm, st) : launch_synthesis<false>(prm, st);
 }
 
 cudaError_t launch_ring_analysis(const RingParams &prm, cudaStream_t st) {
@@ -833,12 +842,6 @@ cudaError_t launch_ring_analysis(const RingParams &prm, cudaStream_t st) {
     case 256: return launch_rings(k_ring_analysis<256>, 256, prm, st);
     default: return launch_rings(k_ring_analysis<kRingThreads>, kRingThreads, prm, st);
   }
-}
-
-__global__ void k_residual(const double *__restrict__ a, const double *__restrict__ b, double *__restrict__ y,
-                           int64_t n) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    y[i] = a[i] - b[i];
 }
 
 __global__ void k_accumulate(const double *__restrict__ x, double *__restrict__ y, int64_t n) {
@@ -868,12 +871,6 @@ cudaError_t launch_shard_exchange(const int64_t *tab, int64_t nrings, int32_t mc
   if (n <= 0) return cudaSuccess;
   k_shard_exchange<<<(unsigned)std::min<int64_t>((n + 7) / 8, 8192), 256, 0, st>>>(tab, nrings, mcount, nvecs, src,
                                                                                      dst, gather);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_residual(const double *a, const double *b, double *y, int64_t n, cudaStream_t st) {
-  if (n <= 0) return cudaSuccess;
-  k_residual<<<(unsigned)std::min<int64_t>((n + 255) / 256, 8192), 256, 0, st>>>(a, b, y, n);
   return cudaGetLastError();
 }
 
