@@ -32,6 +32,7 @@
 #include <algorithm>
 
 #include "kernels.h"
+#include "launch.cuh"
 #include "plan.h"
 
 namespace wm {
@@ -148,6 +149,7 @@ __global__ void __launch_bounds__(kDirectThr, direct_ctas(NV * C)) k_direct_a2m(
 #pragma unroll
       for (int v = 0; v < NV; ++v) acc[j][v] = 0.0;
     }
+    grid_wait();  // the alm, and the readers of q
     if (T.kstart < R) fetch(T.kstart, s_chunk[0]);
     w0 = __reduce_min_sync(0xffffffffu, w0);
     wf = __reduce_max_sync(0xffffffffu, wf);
@@ -277,6 +279,7 @@ __global__ void __launch_bounds__(kDirectThr, NT == 2 ? 3 : 4) k_direct_m2a(Dire
       s_ab[e] = r < R ? p.ab[G.coef + r] : make_double2(0.0, 0.0);
     }
     __syncthreads();
+    grid_wait();  // q~ or X, and the readers of the alm
     const DevDirectCol *cols = p.cols + G.cols;
     const double2 *seeds = p.seeds + T.seeds + lane;
     const int ncg = (T.nact + 3) >> 2, nfull = T.nfull >> 2, r0 = T.row0 + g * S;
@@ -467,9 +470,7 @@ __global__ void k_direct_setup(DirectParams p, const DevGCol *gcols, const doubl
 
 template <int NV>
 static cudaError_t a2m(const DirectParams &p, int width, int npass, int grid, cudaStream_t st) {
-  if (width) k_direct_a2m<NV, 2><<<grid, kDirectThr, 0, st>>>(p, npass);
-  else k_direct_a2m<NV, 1><<<grid, kDirectThr, 0, st>>>(p, npass);
-  return cudaGetLastError();
+  return launch_overlapped(width ? k_direct_a2m<NV, 2> : k_direct_a2m<NV, 1>, grid, kDirectThr, 0, st, p, npass);
 }
 
 cudaError_t launch_direct_a2m(DirectParams p, const DevDirectTileA *const (&tiles)[2], const int32_t (&ntiles)[2],
@@ -510,9 +511,7 @@ cudaError_t launch_direct_m2a(const DirectParams &p, int max_ctas, cudaStream_t 
   const int64_t units = (int64_t)p.ntiles_b * npass;
   if (units <= 0) return cudaSuccess;
   const int grid = (int)std::min<int64_t>(units, max_ctas > 0 ? max_ctas : INT_MAX);
-  if (wide) k_direct_m2a<2><<<grid, kDirectThr, 0, st>>>(p, npass);
-  else k_direct_m2a<1><<<grid, kDirectThr, 0, st>>>(p, npass);
-  return cudaGetLastError();
+  return launch_overlapped(wide ? k_direct_m2a<2> : k_direct_m2a<1>, grid, kDirectThr, 0, st, p, npass);
 }
 
 cudaError_t launch_direct_setup(const DirectParams &p, const DevGCol *gcols, const double *f64, DevDirectCol *cols,

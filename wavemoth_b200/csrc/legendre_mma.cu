@@ -21,6 +21,7 @@
 #include <algorithm>
 
 #include "kernels.h"
+#include "launch.cuh"
 #include "plan.h"
 
 namespace wm {
@@ -100,6 +101,7 @@ __global__ void __launch_bounds__(kThr) k_a2m_level(FastParams p, int npass) {
     const DevPair P = p.pairs[U.pair];
     const double *X = p.xbuf + M.xrow * p.nvecs + v0;
     double *q = p.q + (int64_t)(2 * M.m + M.odd) * p.q_mstride + (int64_t)P.out_left * p.q_rstride + v0;
+    grid_wait();  // X, and the readers of q
     for (int e = threadIdx.x; e < (P.kT + P.kB) * NV; e += kThr) {
       const int s = e / NV, v = e % NV, row = s < P.kT ? P.inT + s : P.inB + (s - P.kT);
       xs[s * VP + v] = v < vn ? X[(int64_t)row * p.nvecs + v] : 0.0;
@@ -160,6 +162,7 @@ __global__ void __launch_bounds__(kThr) k_m2a_level(FastParams p, int npass) {
       sperm[z] = p.i32[P.permT + z];
       sperm[P.n + z] = p.i32[P.permB + z];
     }
+    grid_wait();  // q~, and the readers of X
     for (int e = threadIdx.x; e < P.n * NV; e += kThr) {
       const int z = e / NV, v = e % NV;
       qs[z * VP + v] = v < vn ? q[(int64_t)z * p.q_rstride + v] : 0.0;
@@ -245,8 +248,7 @@ cudaError_t launch_level_nt(bool alm2map, const FastParams &p, int max_ctas, cud
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  kernel<<<grid, kThr, smem, st>>>(p, npass);
-  return cudaGetLastError();
+  return launch_overlapped(kernel, grid, kThr, smem, st, p, npass);
 }
 
 }  // namespace

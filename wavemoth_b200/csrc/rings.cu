@@ -66,6 +66,7 @@
 
 #include "plan.h"
 #include "kernels.h"
+#include "launch.cuh"
 
 namespace wm {
 
@@ -516,6 +517,7 @@ __global__ void __launch_bounds__(kThr, kRingThreads / kThr) k_ring_synthesis(Ri
   cplx *phi = plo + kPhaseLo;
   phase_tables(plo, phi, p, c.ring);
   __syncthreads();
+  grid_wait();  // q, and the readers of the map
   // q rows are ring-major: (m, parity) of ring r at row (r (mmax + 1) + m) 2 + parity
   const int64_t half = p.nvecs, qstride = 2 * half;
   const double *qbase = p.q + (int64_t)c.ring * (p.mmax + 1) * qstride + 2 * c.map0;
@@ -639,6 +641,7 @@ __global__ void __launch_bounds__(kThr, kRingThreads / kThr) k_ring_analysis(Rin
   cplx *plo = buf + ((int64_t)M << lg);
   cplx *phi = plo + kPhaseLo;
   phase_tables(plo, phi, p, c.ring);
+  grid_wait();  // the map, and the readers of q~
   const int64_t half = p.nvecs, qstride = 2 * half;
   double *qbase = p.q_out + (int64_t)c.ring * (p.mmax + 1) * qstride + 2 * c.map0;
   const auto rs = radices<false>(M);
@@ -813,8 +816,7 @@ cudaError_t launch_rings(K kernel, int threads, const RingParams &prm, cudaStrea
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, prm.smem);
     if (e != cudaSuccess) return e;
   }
-  kernel<<<prm.ntasks, threads, prm.smem, st>>>(prm);
-  return cudaGetLastError();
+  return launch_overlapped(kernel, prm.ntasks, threads, prm.smem, st, prm);
 }
 
 template <bool kSub>
