@@ -215,6 +215,13 @@ int wavemoth_shard_map2alm_legendre(wavemoth_plan plan, const double *q_recv, do
    has no analysis direction. */
 int wavemoth_plan_set_ring_weights(wavemoth_plan plan, const double *weights);
 
+/* Gradient of a real loss with respect to the alm of alm2map, from its
+   gradient with respect to the map (device pointers, enqueued on `stream`):
+   (npix / 4 pi) c_m map2alm(grad_map), c_0 = 1, c_m = 2, and Im a_l0 = 0,
+   re/im of every (l, m >= 0) entry being independent variables.  Ring
+   weights, if set, apply as in map2alm. */
+int wavemoth_alm2map_backward_device(wavemoth_plan plan, const double *grad_map, double *grad_alm, void *stream);
+
 /* map2alm refined by niter Jacobi iterations, a_{k+1} = a_k +
    map2alm(f - alm2map(a_k)), on device buffers (layouts as
    wavemoth_execute_map2alm_device) on `stream`.  The first call with

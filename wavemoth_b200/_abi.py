@@ -55,6 +55,7 @@ SIGNATURES = {
     "wavemoth_shard_alm2map_rings": (ctypes.c_int, [_vp, _vp, _vp, _vp, _vp]),
     "wavemoth_shard_map2alm_rings": (ctypes.c_int, [_vp, _vp, _vp, _vp, _vp]),
     "wavemoth_shard_map2alm_legendre": (ctypes.c_int, [_vp, _vp, _vp, _vp]),
+    "wavemoth_alm2map_backward_device": (ctypes.c_int, [_vp, _vp, _vp, _vp]),
     "wavemoth_map2alm_iterative_device": (ctypes.c_int, [_vp, _vp, _vp, ctypes.c_int, _vp]),
     # kernel-level hooks (src/legendre_transform.h, src/butterfly.h.in)
     "wavemoth_legendre_transform_auxdata": (None, [_sz, _sz, _sz, _dp]),

@@ -9,7 +9,8 @@ real field,
     map2alm = (4 pi / Npix) W^-1 A^T,   W = diag(c_m), c_0 = 1, c_m = 2,
 
 so the gradients of both directions are one call of the other direction's
-kernels with a per-m weight (no Legendre values are stored: the backward
+kernels with a per-m weight (alm2map's is applied by the kernel that writes
+the alm: Transform.alm2map_backward; no Legendre values are stored: the backward
 pass regenerates them with the same recurrence as the forward pass):
 
     alm2map backward:  grad_alm = (Npix / 4 pi) c_m map2alm(grad_map)
@@ -42,12 +43,7 @@ class _Alm2Map(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_map):
-        T = ctx.transform
-        g = T.map2alm(grad_map.contiguous())
-        w = _m_weights(T.lmax, g.device) * (T.npix / (4.0 * math.pi))
-        g = g * w[:, None]
-        g[: T.lmax + 1] = g[: T.lmax + 1].real.to(torch.complex128)
-        return g, None
+        return ctx.transform.alm2map_backward(grad_map), None
 
 
 class _Map2Alm(torch.autograd.Function):

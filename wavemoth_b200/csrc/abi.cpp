@@ -1079,6 +1079,10 @@ int run_split(wavemoth_plan P, bool alm2map, const double *alm_in, double *alm_o
   return 0;
 }
 
+// What map2alm does with the alm it computes: writes it, adds it, or writes it
+// as the gradient of a real map (rows of m > 0 twice, Im a_l0 zero).
+enum class AlmOut { kWrite, kAdd, kBackward };
+
 // Whether a plan's Legendre step runs on the FP64 units: always without split
 // precision, and with it where that is faster.  The split GEMMs stream six
 // bytes of sliced P per element whatever the number of maps, the FP64 kernels
@@ -1097,9 +1101,8 @@ bool use_direct(wavemoth_plan P) {
 
 // FP64 path: residual products, and the interpolation levels of depth-1
 // matrices after (alm2map) or before them (map2alm).
-// accumulate: map2alm adds to the alm.
 int run_direct(wavemoth_plan P, bool alm2map, const double *alm_in, double *alm_out, const double *q_in,
-               double *q_out, cudaStream_t st, bool accumulate) {
+               double *q_out, cudaStream_t st, AlmOut how) {
   const auto &G = P->img->prog;
   const int nr = (int)G.roots.size(), cap = P->grid_cap > 0 ? 4 * plan_sms(P) : 0;
   int rc = 0;
@@ -1116,7 +1119,8 @@ int run_direct(wavemoth_plan P, bool alm2map, const double *alm_in, double *alm_
   d.alm_out = alm_out;
   d.q_in = q_in;
   d.q = q_out;
-  d.accumulate = accumulate;
+  d.accumulate = how == AlmOut::kAdd;
+  d.backward = how == AlmOut::kBackward;
   if (alm2map) {
     d.aligned = (((uintptr_t)q_out | (uintptr_t)alm_in) & 15) == 0;
     rc = cuda_check(wm::launch_direct_a2m(d, P->d_direct_a, P->ndirect_a, plan_sms(P), cap, st),
@@ -1131,16 +1135,15 @@ int run_direct(wavemoth_plan P, bool alm2map, const double *alm_in, double *alm_
   return rc;
 }
 
-// accumulate (map2alm, where accumulates(P)): adds to the alm.
 int run_legendre(wavemoth_plan P, bool alm2map, const double *alm_in, double *alm_out,
-                 const double *q_in, double *q_out, cudaStream_t st, bool accumulate = false) {
+                 const double *q_in, double *q_out, cudaStream_t st, AlmOut how = AlmOut::kWrite) {
   const auto &G = P->img->prog;
   int sp = span_begin(P, alm2map ? 0 : 1, st);
   int rc = 0;
   if (!use_direct(P)) {
     rc = run_split(P, alm2map, alm_in, alm_out, q_in, q_out, st);
   } else {
-    rc = run_direct(P, alm2map, alm_in, alm_out, q_in, q_out, st, accumulate);
+    rc = run_direct(P, alm2map, alm_in, alm_out, q_in, q_out, st, how);
   }
   if (!rc && P->nslow > 0) {
     wm::LegendreParams p = legendre_params(P);
@@ -1160,8 +1163,9 @@ int run_legendre(wavemoth_plan P, bool alm2map, const double *alm_in, double *al
   return rc;
 }
 
-// Whether the plan's map2alm can add to the alm: every matrix on the FP64 units.
-bool accumulates(wavemoth_plan P) { return use_direct(P) && P->nslow == 0; }
+// Whether the plan's map2alm can do more than write the alm (AlmOut): every
+// matrix on the FP64 units.
+bool weighs_alm(wavemoth_plan P) { return use_direct(P) && P->nslow == 0; }
 
 // scale multiplies the maps (1 for alm2map; 4 pi / npix for the adjoint of
 // map2alm); sub, if given, is what they are subtracted from
@@ -1186,7 +1190,7 @@ int run_alm2map(wavemoth_plan P, const double *alm, double *map, cudaStream_t st
 
 // scale multiplies q~ (4 pi / npix for map2alm; 1 for the adjoint of alm2map)
 int run_map2alm(wavemoth_plan P, const double *map, double *alm, cudaStream_t st, double scale = -1.0,
-                bool accumulate = false) {
+                AlmOut how = AlmOut::kWrite) {
   wm::RingParams r = ring_params(P);
   r.map_in = map;
   r.q_out = P->d_q;
@@ -1199,7 +1203,7 @@ int run_map2alm(wavemoth_plan P, const double *map, double *alm, cudaStream_t st
   P->kernel_launches += r.ntasks > 0;
   span_end(P, sp, st);
   if (rc0) return rc0;
-  return run_legendre(P, false, nullptr, alm, P->d_q, nullptr, st, accumulate);
+  return run_legendre(P, false, nullptr, alm, P->d_q, nullptr, st, how);
 }
 
 // Reads (and clears) the device status word; the stream must be idle.
@@ -1493,13 +1497,26 @@ int wavemoth_plan_set_ring_weights(wavemoth_plan plan, const double *weights) {
   return 0;
 }
 
+int wavemoth_alm2map_backward_device(wavemoth_plan plan, const double *grad_map, double *grad_alm, void *stream) {
+  if (!plan || !grad_alm || !grad_map) return set_error(WAVEMOTH_ERR_ARG, "NULL plan or buffer");
+  cudaStream_t st = (cudaStream_t)stream;
+  const bool fused = weighs_alm(plan);
+  int rc = run_map2alm(plan, grad_map, grad_alm, st, 1.0, fused ? AlmOut::kBackward : AlmOut::kWrite);
+  if (!rc && !fused) {
+    rc = cuda_check(wm::launch_backward_weights(grad_alm, plan->lmax + 1, plan->nalm, plan->nvecs, st),
+                    "backward weights");
+    plan->kernel_launches++;
+  }
+  return finish(plan, rc);
+}
+
 int wavemoth_map2alm_iterative_device(wavemoth_plan plan, const double *map, double *alm, int niter,
                                       void *stream) {
   if (!plan || !alm || !map || niter < 0) return set_error(WAVEMOTH_ERR_ARG, "NULL plan or buffer, or niter < 0");
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t nmap = plan->npix * plan->nmaps, nalm = plan->nalm * plan->nvecs;
   int rc = 0;
-  const bool add = accumulates(plan);
+  const bool add = weighs_alm(plan);
   if (niter > 0 && !plan->d_iter_map) rc = plan->arena.alloc(&plan->d_iter_map, (size_t)nmap, "iteration map buffer");
   if (niter > 0 && !add && !plan->d_iter_alm)
     rc = rc ? rc : plan->arena.alloc(&plan->d_iter_alm, (size_t)nalm, "iteration alm buffer");
@@ -1508,7 +1525,8 @@ int wavemoth_map2alm_iterative_device(wavemoth_plan plan, const double *map, dou
   for (int it = 0; it < niter && !rc; ++it) {
     // a += map2alm(f - alm2map(a))
     rc = run_alm2map(plan, alm, plan->d_iter_map, st, 1.0, map);
-    if (!rc) rc = run_map2alm(plan, plan->d_iter_map, add ? alm : plan->d_iter_alm, st, -1.0, add);
+    if (!rc) rc = run_map2alm(plan, plan->d_iter_map, add ? alm : plan->d_iter_alm, st, -1.0,
+                              add ? AlmOut::kAdd : AlmOut::kWrite);
     if (rc || add) continue;
     rc = cuda_check(wm::launch_accumulate(plan->d_iter_alm, alm, nalm, st), "accumulate");
     plan->kernel_launches++;

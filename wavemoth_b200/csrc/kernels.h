@@ -84,6 +84,7 @@ struct DirectParams {
   double *xbuf;
   int32_t aligned;              // the alm and q are 16-byte aligned (alm2map)
   int32_t accumulate;           // map2alm: adds to the alm
+  int32_t backward;             // map2alm: rows of m > 0 twice, imaginary parts of m = 0 zero
 };
 
 // max_ctas > 0 bounds the grid (the units are then walked by fewer CTAs);
@@ -226,6 +227,8 @@ cudaError_t launch_strided_copy(double *dst, int64_t dpitch, const double *src, 
                                 int64_t rows, cudaStream_t st);
 
 cudaError_t launch_ring_synthesis(const RingParams &prm, cudaStream_t st);
+// alm rows [0, split) with zero imaginary parts, the others twice (rows of nvecs doubles).
+cudaError_t launch_backward_weights(double *alm, int64_t split, int64_t rows, int32_t nvecs, cudaStream_t st);
 // y += x (n doubles).
 cudaError_t launch_accumulate(const double *x, double *y, int64_t n, cudaStream_t st);
 // m-sharded plans: moves the 2 nvecs doubles of every (ring of this part,

@@ -410,8 +410,9 @@ __global__ void __launch_bounds__(kDirectThr, NT == 2 ? 3 : 4) k_direct_m2a(Dire
           const int r = e >> 3, v = e & 7, at = 8 * (r % S) + r / S;
           if (8 * nt + v < vn) {
             double *to = dst + 2 * (int64_t)r * p.nvecs + 8 * nt + v;
-            const double a = ((s_red[0][at][v] + s_red[1][at][v]) + (s_red[2][at][v] + s_red[3][at][v])) *
-                             p.scale[G.coef + T.row0 + r];
+            double a = ((s_red[0][at][v] + s_red[1][at][v]) + (s_red[2][at][v] + s_red[3][at][v])) *
+                       p.scale[G.coef + T.row0 + r];
+            if (p.backward) a = M.m ? 2.0 * a : (v & 1) ? 0.0 : a;
             *to = p.accumulate ? *to + a : a;
           }
         }

@@ -846,6 +846,11 @@ cudaError_t launch_ring_analysis(const RingParams &prm, cudaStream_t st) {
   }
 }
 
+__global__ void k_backward_weights(double *__restrict__ alm, int64_t split, int64_t n) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    alm[i] = i >= split ? 2.0 * alm[i] : (i & 1) ? 0.0 : alm[i];
+}
+
 __global__ void k_accumulate(const double *__restrict__ x, double *__restrict__ y, int64_t n) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     y[i] += x[i];
@@ -873,6 +878,13 @@ cudaError_t launch_shard_exchange(const int64_t *tab, int64_t nrings, int32_t mc
   if (n <= 0) return cudaSuccess;
   k_shard_exchange<<<(unsigned)std::min<int64_t>((n + 7) / 8, 8192), 256, 0, st>>>(tab, nrings, mcount, nvecs, src,
                                                                                      dst, gather);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_backward_weights(double *alm, int64_t split, int64_t rows, int32_t nvecs, cudaStream_t st) {
+  const int64_t n = rows * nvecs;
+  if (n <= 0) return cudaSuccess;
+  k_backward_weights<<<(unsigned)std::min<int64_t>((n + 255) / 256, 8192), 256, 0, st>>>(alm, split * nvecs, n);
   return cudaGetLastError();
 }
 

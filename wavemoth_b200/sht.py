@@ -84,6 +84,19 @@ class Transform:
             raise WavemothError("map2alm failed (%d): %s" % (rc, last_error()))
         return out
 
+    def alm2map_backward(self, grad_map, out=None):
+        """Gradient of a loss with respect to the alm of alm2map, from its
+        gradient with respect to the map: (npix / 4 pi) c_m map2alm(grad_map),
+        c_0 = 1, c_m = 2, with Im a_l0 zero (re/im as independent variables)."""
+        grad_map = self._check_map(grad_map)
+        if out is None:
+            out = torch.empty((self.nalm, self.nmaps), dtype=torch.complex128, device=grad_map.device)
+        rc = _native.lib().wavemoth_alm2map_backward_device(
+            self._plans["map2alm"], grad_map.data_ptr(), out.data_ptr(), self._stream())
+        if rc != 0:
+            raise WavemothError("alm2map backward failed (%d): %s" % (rc, last_error()))
+        return out
+
     def set_ring_weights(self, weights):
         """Quadrature weights of the 2 Nside ring pairs (equator first) used by
         map2alm (wavemoth_b200.weights.ring_weights), or None for unit
