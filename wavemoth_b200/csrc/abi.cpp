@@ -151,7 +151,7 @@ struct _wavemoth_plan : ImageRefs {
   int8_t *d_planes = nullptr;
   int32_t *d_status = nullptr;
   wm::DevRingTask *d_ring_tasks = nullptr;
-  int32_t ring_ntasks = 0, ring_smem = 0, ring_threads = 0;
+  int32_t ring_ntasks = 0, ring_smem = 0, ring_threads = 0, ring_short = 0;
   double *d_alm = nullptr, *d_map = nullptr, *d_q = nullptr, *d_scratch = nullptr;
   double *d_ring_weights = nullptr;           // per ring pair (null: unweighted analysis)
   double *d_ring_weights_buf = nullptr;
@@ -225,7 +225,7 @@ struct RingTable {
   int32_t twlen = 4;         // largest power-of-two table length needed
   int32_t max_bluestein = 0;
   int32_t smem = 0;
-  int32_t threads = 0;
+  int32_t threads = 0, short_rings = 0;
   int32_t nphase_hi = 1;
   int64_t max_cta_cplx = 0;  // largest transform buffer of one CTA
 };
@@ -278,7 +278,19 @@ RingTable ring_table(int nside, int nmaps, int mmax, bool one_side = false) {
     while (len < ((N & (N - 1)) ? 2 * N - 1 : N)) len <<= 1;
     longest = std::max(longest, 2 * len);
   }
-  const int buffer = std::min(wm::kRingBufferCplx, std::max(2048, nmaps >= 16 ? 2 * longest : longest));
+  //
+  // The shortest rings (up to nside 64; by the ring length alone, so that a map
+  // gives the same bits whatever is beside it) run in passes of radix 4: a
+  // radix-16 butterfly of theirs keeps one thread busy for longer than the
+  // passes it saves take.  A quarter of the points per CTA then feed every
+  // thread; with 16 maps and more, as many as before.  Measured, alm2map /
+  // map2alm, radix 16 -> 4, us: nside 32, 3 maps 14.3 / 12.6 -> 14.0 / 10.4, 32
+  // maps 23.2 / 22.1 -> 23.6 / 19.9; nside 64, 1 map 15.3 / 15.4 -> 14.9 / 11.2, 8
+  // maps 20.1 / 20.0 -> 19.6 / 17.8, 32 maps 43.8 / 43.4 -> 44.9 / 43.1; nside
+  // 256, 1 map 56 / 100 -> 60 / 103.
+  const bool short_rings = longest <= 512;
+  const int least = short_rings ? 512 : 2048, most = short_rings ? 4 * longest : 2 * longest;
+  const int buffer = std::min(wm::kRingBufferCplx, std::max(least, nmaps >= 16 ? most : longest));
   struct Item { double cost; wm::DevRingTask t; int64_t cplx; };
   std::vector<Item> items;
   for (int r = 0; r < 2 * nside; ++r) {
@@ -332,6 +344,7 @@ RingTable ring_table(int nside, int nmaps, int mmax, bool one_side = false) {
   }
   T.smem = T.tasks.empty() ? 0 : wm::ring_cta_smem(need, T.nphase_hi);
   T.threads = need > 4096 ? 512 : need > 2048 ? 256 : 128;  // 16 points per thread
+  T.short_rings = short_rings;
   return T;
 }
 
@@ -874,6 +887,7 @@ wavemoth_plan make_plan(bool analysis, int Nside, int lmax, int mmax, int nmaps,
     P->ring_ntasks = (int32_t)RT.tasks.size();
     P->ring_smem = RT.smem;
     P->ring_threads = RT.threads;
+    P->ring_short = RT.short_rings;
     rc = rc ? rc : upload(A, &P->d_ring_tasks, RT.tasks, "ring work list");
   }
   if (img->split) {
@@ -976,6 +990,7 @@ wm::RingParams ring_params(wavemoth_plan P) {
   r.ntasks = P->ring_ntasks;
   r.smem = P->ring_smem;
   r.threads = P->ring_threads;
+  r.short_rings = P->ring_short;
   r.nphase_hi = P->nphase_hi;
   r.phases = P->d_phases;
   return r;
@@ -1586,6 +1601,7 @@ int wavemoth_plan_set_hemisphere_mode(wavemoth_plan plan, int one_side) {
   plan->ring_ntasks = (int32_t)RT.tasks.size();
   plan->ring_smem = RT.smem;
   plan->ring_threads = RT.threads;
+  plan->ring_short = RT.short_rings;
   return 0;
 }
 

@@ -214,6 +214,7 @@ struct RingParams {
   int32_t ntasks;
   int32_t smem;           // bytes
   int32_t threads;        // per CTA: 128, 256 or 512
+  int32_t short_rings;    // CTAs of 128 threads: passes of radix 4 instead of 16
   int32_t nphase_hi;      // entries of the coarse phase table (mmax / 64 + 1)
   // per ring pair, kPhaseLo + nphase_hi phase factors (fine then coarse
   // table), computed at plan creation

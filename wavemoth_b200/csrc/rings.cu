@@ -14,7 +14,8 @@
 //   ring[2s] = Re z[s], ring[2s+1] = Im z[s],  z = IDFT_N(Z)
 // and the analysis r2c uses the mirror identity.
 //
-// Length-N transforms, in place in shared memory, as passes of radix 16 (and
+// Length-N transforms, in place in shared memory, as passes of radix 16 (4 for
+// the shortest rings, RingParams::short_rings, with the same structure; and
 // one last decimation-in-frequency pass of radix 2, 4 or 8 when log2 of the
 // length is not a multiple of 4); a pass loads 16 points per butterfly into
 // registers and runs four radix-2 stages there.  The first radix-16 pass of
@@ -72,7 +73,8 @@ namespace wm {
 
 namespace {
 
-constexpr int kRadixLog = 4;           // largest pass radix 2^kRadixLog
+constexpr int kRadixLog = 4;           // pass radix 2^kRadixLog of all but the shortest transforms
+constexpr int kShortRadixLog = 2;      // theirs
 constexpr int kRingThreads = 512;      // 16 points per thread of a kRingBufferCplx buffer
 constexpr int kPhaseLo = kRingPhaseLo;  // e^{i m phi0} = hi[m / 64] * lo[m % 64]
 
@@ -207,10 +209,11 @@ namespace {
 
 // Shared arguments of the passes of one CTA of kWarps warps: the twiddle
 // table (2^lgtw entries), the transform length M and the log2 of the lanes.
-template <int kWarps>
+template <int kWarps, int kRL>
 struct FftCtx {
   static constexpr int warps = kWarps;
-  static_assert(16 % kWarps == 0, "warp-local passes divide the 16 blocks of a radix-16 pass among the warps");
+  static constexpr int radix_log = kRL;
+  static_assert((1 << kRL) % kWarps == 0, "warp-local passes divide the blocks of the first pass among the warps");
   const double2 *tw;
   int lgtw;
   int M;
@@ -232,8 +235,8 @@ __device__ __forceinline__ void for_butterflies(const Ctx &f, int wl, BodyF body
     for (int t = threadIdx.x; t < nbf; t += blockDim.x) body(t >> f.lg, t & gm);
     __syncthreads();
   } else {
-    // warp w owns the blocks [w k, (w + 1) k): nblk >= 16 blocks (a power of
-    // two) over the CTA's warps; its lanes run over (block, butterfly)
+    // warp w owns the blocks [w k, (w + 1) k): a power of two of blocks, at
+    // least the CTA's warps; its lanes run over (block, butterfly)
     const int k = (f.M >> wl) / Ctx::warps, warp = threadIdx.x >> 5;
     const int lp = wl - LR + f.lg;  // log2 of the butterflies of one block, all lanes
     for (int i = threadIdx.x & 31; i < (k << lp); i += 32) {
@@ -269,27 +272,21 @@ __device__ __forceinline__ void fft_pass(const Ctx &f, int lglen, int wl, LoadF 
 
 template <int SIGN, bool DIF, class Ctx, class LoadF, class StoreF>
 __device__ __forceinline__ void fft_pass_r(const Ctx &f, int R, int lglen, int wl, LoadF load, StoreF store) {
-  switch (R) {
-    case 2: fft_pass<2, SIGN, DIF, false>(f, lglen, wl, load, store); break;
-    case 4: fft_pass<4, SIGN, DIF, false>(f, lglen, wl, load, store); break;
-    case 8:
-      if (kRadixLog > 3) {
-        fft_pass<8, SIGN, DIF, false>(f, lglen, wl, load, store);
-        break;
-      }
-      [[fallthrough]];
-    default: fft_pass<(1 << kRadixLog), SIGN, DIF, false>(f, lglen, wl, load, store); break;
-  }
+  constexpr int kRL = Ctx::radix_log;
+  if (R == 2) fft_pass<2, SIGN, DIF, false>(f, lglen, wl, load, store);
+  else if (kRL > 2 && R == 4) fft_pass<4, SIGN, DIF, false>(f, lglen, wl, load, store);
+  else if (kRL > 3 && R == 8) fft_pass<8, SIGN, DIF, false>(f, lglen, wl, load, store);
+  else fft_pass<(1 << kRL), SIGN, DIF, false>(f, lglen, wl, load, store);
 }
 
 // The first pass of Bluestein's forward transform (the input is zero from N
 // <= M / 2 on) and the last of its inverse (only the first N results are
-// wanted): radix 16 over the whole sequence, as the first of several DIF
+// wanted): the full radix over the whole sequence, as the first of several DIF
 // passes always is, with half of the reads or writes and of one stage left
 // out.
 template <int SIGN, bool DIF, class Ctx, class LoadF, class StoreF>
 __device__ __forceinline__ void bluestein_end(const Ctx &f, int lglen, LoadF load, StoreF store) {
-  fft_pass<(1 << kRadixLog), SIGN, DIF, true>(f, lglen, 0, load, store);
+  fft_pass<(1 << Ctx::radix_log), SIGN, DIF, true>(f, lglen, 0, load, store);
 }
 
 // Middle of Bluestein's convolution on blocks of R points (R = the last DIF
@@ -332,51 +329,43 @@ __device__ __forceinline__ void bluestein_mid_r(const Ctx &f, const cplx *F, int
 template <class Ctx, class LoadF, class StoreF>
 __device__ __forceinline__ void bluestein_mid(const Ctx &f, int R, const cplx *F, int fsign, int wl, LoadF load,
                                               StoreF store) {
-  switch (R) {
-    case 2: bluestein_mid_r<2>(f, F, fsign, wl, load, store); break;
-    case 4: bluestein_mid_r<4>(f, F, fsign, wl, load, store); break;
-    case 8:
-      if (kRadixLog > 3) {
-        bluestein_mid_r<8>(f, F, fsign, wl, load, store);
-        break;
-      }
-      [[fallthrough]];
-    default: bluestein_mid_r<(1 << kRadixLog)>(f, F, fsign, wl, load, store); break;
-  }
+  constexpr int kRL = Ctx::radix_log;
+  if (R == 2) bluestein_mid_r<2>(f, F, fsign, wl, load, store);
+  else if (kRL > 2 && R == 4) bluestein_mid_r<4>(f, F, fsign, wl, load, store);
+  else if (kRL > 3 && R == 8) bluestein_mid_r<8>(f, F, fsign, wl, load, store);
+  else bluestein_mid_r<(1 << kRL)>(f, F, fsign, wl, load, store);
 }
 
-// Pass radices of a length-M transform in DIF order: the radix-16 passes
-// and one pass of radix 2^(log2 M mod 4) (if above 1), first or last.  DIT
+// Pass radices of a length-M transform in DIF order: passes of radix 2^kRL
+// and one pass of radix 2^(log2 M mod kRL) (if above 1), first or last.  DIT
 // runs them in reverse order.  Once the passes before p have cut every
-// lane into at least 16 blocks (one or more per warp of the CTA), pass p and
-// the later DIF passes (the earlier DIT passes) run warp-local on the blocks
-// of pass p0 (for_butterflies).  Computed per pass (no per-thread arrays,
-// which would live in local memory).
-template <bool kSmallFirst>
+// lane into at least one block per warp of the CTA, pass p and the later DIF
+// passes (the earlier DIT passes) run warp-local on the blocks of pass p0
+// (for_butterflies).  Computed per pass (no per-thread arrays, which would
+// live in local memory).
+template <bool kSmallFirst, int kRL>
 struct Radices {
   int lgM;  // log2 M
-  int r0;   // log2 M mod 4: log2 of the small radix, 0 if none
+  int r0;   // log2 M mod kRL: log2 of the small radix, 0 if none
   int n;    // number of passes
   // radix of DIF pass p
-  __device__ __forceinline__ int r(int p) const {
-    return (r0 && p == (kSmallFirst ? 0 : n - 1)) ? 1 << r0 : 1 << kRadixLog;
-  }
+  __device__ __forceinline__ int r(int p) const { return (r0 && p == (kSmallFirst ? 0 : n - 1)) ? 1 << r0 : 1 << kRL; }
   // log2 of the block length of DIF pass p (the DIT pass mirroring it has the same)
   __device__ __forceinline__ int lgl(int p) const {
-    return lgM - kRadixLog * p + ((kSmallFirst && r0 && p > 0) ? kRadixLog - r0 : 0);
+    return lgM - kRL * p + ((kSmallFirst && r0 && p > 0) ? kRL - r0 : 0);
   }
-  // first warp-local DIF pass: the first after a radix-16 pass
+  // first warp-local DIF pass: the first after a pass of the full radix
   __device__ __forceinline__ int p0() const { return (kSmallFirst && r0) ? 2 : 1; }
   // log2 of the per-lane block a warp owns in pass p (0: the whole CTA runs the pass)
   __device__ __forceinline__ int wl(int p) const { return (p >= p0() && p < n) ? lgl(p0()) : 0; }
 };
 
-template <bool kSmallFirst>
-__device__ __forceinline__ Radices<kSmallFirst> radices(int M) {
-  Radices<kSmallFirst> s;
+template <bool kSmallFirst, int kRL>
+__device__ __forceinline__ Radices<kSmallFirst, kRL> radices(int M) {
+  Radices<kSmallFirst, kRL> s;
   s.lgM = ilog2(M);
-  s.r0 = s.lgM % kRadixLog;
-  s.n = s.lgM / kRadixLog + (s.r0 ? 1 : 0);
+  s.r0 = s.lgM % kRL;
+  s.n = s.lgM / kRL + (s.r0 ? 1 : 0);
   return s;
 }
 
@@ -507,7 +496,7 @@ __device__ __forceinline__ void alias_sums(const double *qg, int j, int n, int m
 }
 
 // kSub: writes map_sub - map instead of the map.
-template <int kThr, bool kSub>
+template <int kThr, int kRL, bool kSub>
 __global__ void __launch_bounds__(kThr, kRingThreads / kThr) k_ring_synthesis(RingParams p) {
   extern __shared__ double smem_d[];
   const RingCta c = ring_cta(p, blockIdx.x);
@@ -523,8 +512,8 @@ __global__ void __launch_bounds__(kThr, kRingThreads / kThr) k_ring_synthesis(Ri
   const double *qbase = p.q + (int64_t)c.ring * (p.mmax + 1) * qstride + 2 * c.map0;
   // the aliasing sums stop at the ring's m limit (null: every m)
   const int mlim = p.ring_mend ? p.ring_mend[c.ring] - 1 : p.mmax;
-  const auto rs = radices<false>(M);
-  const FftCtx<kThr / 32> fx{p.twiddles, ilog2(p.twlen), M, lg};
+  const auto rs = radices<false, kRL>(M);
+  const FftCtx<kThr / 32, kRL> fx{p.twiddles, ilog2(p.twlen), M, lg};
   const cplx *F = reinterpret_cast<const cplx *>(p.filters) + c.R.filter;
   const double inv = (c.pow2 ? 1.0 : 1.0 / (double)M) * p.map_scale;
   const int gmm = (1 << c.lgm) - 1;
@@ -632,7 +621,7 @@ __global__ void __launch_bounds__(kThr, kRingThreads / kThr) k_ring_synthesis(Ri
   }
 }
 
-template <int kThr>
+template <int kThr, int kRL>
 __global__ void __launch_bounds__(kThr, kRingThreads / kThr) k_ring_analysis(RingParams p) {
   extern __shared__ double smem_d[];
   const RingCta c = ring_cta(p, blockIdx.x);
@@ -644,8 +633,8 @@ __global__ void __launch_bounds__(kThr, kRingThreads / kThr) k_ring_analysis(Rin
   grid_wait();  // the map, and the readers of q~
   const int64_t half = p.nvecs, qstride = 2 * half;
   double *qbase = p.q_out + (int64_t)c.ring * (p.mmax + 1) * qstride + 2 * c.map0;
-  const auto rs = radices<false>(M);
-  const FftCtx<kThr / 32> fx{p.twiddles, ilog2(p.twlen), M, lg};
+  const auto rs = radices<false, kRL>(M);
+  const FftCtx<kThr / 32, kRL> fx{p.twiddles, ilog2(p.twlen), M, lg};
   const cplx *F = reinterpret_cast<const cplx *>(p.filters) + c.R.filter;
   const double inv = c.pow2 ? 1.0 : 1.0 / (double)M;
   const int gmm = (1 << c.lgm) - 1;
@@ -801,8 +790,8 @@ __global__ void __launch_bounds__(kRingThreads) k_bluestein_filters(RingParams p
   __syncthreads();
   auto sload = [&](int i, int g) -> cplx { return buf[at(i, g, 0)]; };
   auto sstore = [&](int i, int g, cplx v) { buf[at(i, g, 0)] = v; };
-  const auto rs = radices<true>(M);
-  const FftCtx<kRingThreads / 32> fx{p.twiddles, ilog2(p.twlen), M, 0};
+  const auto rs = radices<true, kRadixLog>(M);
+  const FftCtx<kRingThreads / 32, kRadixLog> fx{p.twiddles, ilog2(p.twlen), M, 0};
   for (int ps = 0; ps < rs.n; ++ps)
     fft_pass_r<-1, true>(fx, rs.r(ps), rs.lgl(ps), 0, sload, sstore);
   cplx *F = reinterpret_cast<cplx *>(p.filters_out) + R.filter;
@@ -822,9 +811,11 @@ cudaError_t launch_rings(K kernel, int threads, const RingParams &prm, cudaStrea
 template <bool kSub>
 cudaError_t launch_synthesis(const RingParams &prm, cudaStream_t st) {
   switch (prm.threads) {
-    case 128: return launch_rings(k_ring_synthesis<128, kSub>, 128, prm, st);
-    case 256: return launch_rings(k_ring_synthesis<256, kSub>, 256, prm, st);
-    default: return launch_rings(k_ring_synthesis<kRingThreads, kSub>, kRingThreads, prm, st);
+    case 128:
+      return launch_rings(prm.short_rings ? k_ring_synthesis<128, kShortRadixLog, kSub>
+                                          : k_ring_synthesis<128, kRadixLog, kSub>, 128, prm, st);
+    case 256: return launch_rings(k_ring_synthesis<256, kRadixLog, kSub>, 256, prm, st);
+    default: return launch_rings(k_ring_synthesis<kRingThreads, kRadixLog, kSub>, kRingThreads, prm, st);
   }
 }
 
@@ -840,9 +831,11 @@ cudaError_t launch_ring_synthesis(const RingParams &prm, cudaStream_t st) {
 
 cudaError_t launch_ring_analysis(const RingParams &prm, cudaStream_t st) {
   switch (prm.threads) {
-    case 128: return launch_rings(k_ring_analysis<128>, 128, prm, st);
-    case 256: return launch_rings(k_ring_analysis<256>, 256, prm, st);
-    default: return launch_rings(k_ring_analysis<kRingThreads>, kRingThreads, prm, st);
+    case 128:
+      return launch_rings(prm.short_rings ? k_ring_analysis<128, kShortRadixLog> : k_ring_analysis<128, kRadixLog>,
+                          128, prm, st);
+    case 256: return launch_rings(k_ring_analysis<256, kRadixLog>, 256, prm, st);
+    default: return launch_rings(k_ring_analysis<kRingThreads, kRadixLog>, kRingThreads, prm, st);
   }
 }
 
