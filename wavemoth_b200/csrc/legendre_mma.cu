@@ -75,6 +75,11 @@ __device__ __forceinline__ void level_tile(const double *a, int lda, int rows, i
   }
 }
 
+// Starts the way of n doubles into the L2 cache.
+__device__ __forceinline__ void prefetch_l2(const double *x, int n) {
+  for (int e = 16 * threadIdx.x; e < n; e += 16 * kThr) asm volatile("prefetch.global.L2 [%0];" ::"l"(x + e));
+}
+
 // ------------------------------------------------------------------------
 // alm2map level: one unit = one depth-1 root and 8 NT vectors.  q rows are the
 // sum of the T and the B block's rows; a block's k skeleton rows are its X
@@ -85,8 +90,10 @@ __device__ __forceinline__ void level_tile(const double *a, int lda, int rows, i
 //
 // Bound: the latency of a root's small products (about 64 x 64 per block), so
 // several CTAs per SM.  Reading W[z][s] through the row map element by element
-// took 142 us at nside 256, 7 maps, every matrix with one level, this 93
-// (map2alm 224 -> 84).
+// took 142 us at nside 256, 7 maps, every matrix with one level, this 85
+// (map2alm 224 -> 84): 93 before the interpolants were started on their way
+// to the L2 cache ahead of the X rows and the permutations read once (the
+// same in map2alm, which has its operand's rows to wait for first, lost 4).
 // ------------------------------------------------------------------------
 template <int NT>
 __global__ void __launch_bounds__(kThr) k_a2m_level(FastParams p, int npass) {
@@ -94,6 +101,7 @@ __global__ void __launch_bounds__(kThr) k_a2m_level(FastParams p, int npass) {
   extern __shared__ double level_smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g4 = lane >> 2, t4 = lane & 3;
   double *xs = level_smem, *ys = level_smem + p.max_root_k * VP;
+  int32_t *sperm = reinterpret_cast<int32_t *>(ys + p.max_root_n * VP);  // T, then B
   for (int unit = blockIdx.x; unit < p.nroots * npass; unit += gridDim.x) {
     const DevRootUnit U = p.roots[unit / npass];
     const int v0 = (unit % npass) * NV, vn = min(NV, p.nvecs - v0);
@@ -101,6 +109,12 @@ __global__ void __launch_bounds__(kThr) k_a2m_level(FastParams p, int npass) {
     const DevPair P = p.pairs[U.pair];
     const double *X = p.xbuf + M.xrow * p.nvecs + v0;
     double *q = p.q + (int64_t)(2 * M.m + M.odd) * p.q_mstride + (int64_t)P.out_left * p.q_rstride + v0;
+    prefetch_l2(p.f64 + P.ipT_t, (P.n - P.kT) * P.kT);
+    prefetch_l2(p.f64 + P.ipB_t, (P.n - P.kB) * P.kB);
+    for (int z = threadIdx.x; z < P.n; z += kThr) {
+      sperm[z] = p.i32[P.permT + z];
+      sperm[P.n + z] = p.i32[P.permB + z];
+    }
     grid_wait();  // X, and the readers of q
     for (int e = threadIdx.x; e < (P.kT + P.kB) * NV; e += kThr) {
       const int s = e / NV, v = e % NV, row = s < P.kT ? P.inT + s : P.inB + (s - P.kT);
@@ -111,17 +125,16 @@ __global__ void __launch_bounds__(kThr) k_a2m_level(FastParams p, int npass) {
     for (int part = 0; part < 2; ++part) {
       const int k = part ? P.kB : P.kT, m = P.n - k;
       const double *xp = xs + (part ? P.kT * VP : 0), *ip = p.f64 + (part ? P.ipB_t : P.ipT_t);
-      const int32_t *perm = p.i32 + (part ? P.permB : P.permT);
       auto put = [&](int z, int v, double y) {
         double *at = ys + z * VP + v;
         *at = part ? *at + y : y;
       };
-      for (int e = threadIdx.x; e < k * NV; e += kThr) put(perm[e / NV], e % NV, xp[e / NV * VP + e % NV]);
+      for (int e = threadIdx.x; e < k * NV; e += kThr) put(sperm[part * P.n + e / NV], e % NV, xp[e / NV * VP + e % NV]);
       for (int mt = warp; 8 * mt < m; mt += kThr / 32) {
         double acc[NT][2];
         level_tile<NT>(ip, m, m, k, mt, [&](int j) { return xp + j * VP; }, acc);
         if (8 * mt + g4 < m) {
-          const int z = perm[k + 8 * mt + g4];
+          const int z = sperm[part * P.n + k + 8 * mt + g4];
 #pragma unroll
           for (int nt = 0; nt < NT; ++nt) {
             put(z, 8 * nt + 2 * t4, acc[nt][0]);
@@ -233,8 +246,8 @@ __global__ void k_seeds(FastParams p) {
 
 template <int NT>
 size_t level_smem(bool alm2map, const FastParams &p) {
-  return alm2map ? (size_t)(p.max_root_k + p.max_root_n) * kLevelPitch<NT> * sizeof(double)
-                 : (size_t)p.max_root_n * (kLevelPitch<NT> * sizeof(double) + 2 * sizeof(int32_t));
+  const size_t rows = p.max_root_n + (alm2map ? p.max_root_k : 0);
+  return rows * kLevelPitch<NT> * sizeof(double) + (size_t)p.max_root_n * 2 * sizeof(int32_t);
 }
 
 template <int NT>
