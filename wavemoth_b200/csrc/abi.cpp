@@ -528,7 +528,8 @@ int build_image(DeviceImage &I, int nside, int mmax, unsigned flags) {
     rc = rc ? rc : upload(A, &I.d_order_slow, slow, "slow order");
   }
   rc = rc ? rc : upload(A, &I.d_groups, G.groups, "groups");
-  rc = rc ? rc : upload(A, &I.d_gcols, G.gcols, "group columns");
+  // (the FP64 path's tables are made from the group columns and replace them)
+  if (flags & WAVEMOTH_PRECISION_SPLIT) rc = rc ? rc : upload(A, &I.d_gcols, G.gcols, "group columns");
   rc = rc ? rc : upload(A, &I.d_roots, G.roots, "roots");
   I.split = (flags & WAVEMOTH_PRECISION_SPLIT) != 0;
   if (!I.split) rc = rc ? rc : build_direct(I);
@@ -589,20 +590,31 @@ void alloc_residual_slices(DeviceImage &I, int64_t plan_bytes, unsigned flags) {
 // tables, recurrence seeds, split scales and slices.
 int init_image(wavemoth_plan P) {
   auto &G = P->img->prog;
-  int rc = 0;
-  {
+  // the uploads went through the default stream, which the plan's does not wait for
+  int rc = cuda_check(cudaStreamSynchronize(0), "image upload");
+  if (!rc) {
     wm::RingParams rp = ring_params(P);
     rc = cuda_check(wm::launch_ring_setup(rp, P->d_twiddles, P->max_bluestein ? P->d_filters : nullptr,
                                           P->d_ring_aux, P->d_phases, P->stream), "ring setup launch");
     if (!rc) rc = cuda_check(cudaStreamSynchronize(P->stream), "ring setup");
   }
   if (!rc && P->direct && !G.gcols.empty()) {
-    rc = cuda_check(cudaMemsetAsync(P->d_direct_seeds, 0, std::max<int64_t>(G.direct_seeds, 1) * sizeof(double2),
-                                    P->stream), "segment seeds");
+    wm::DevGCol *gcols = nullptr;
+    if (!P->d_gcols) {
+      const size_t bytes = G.gcols.size() * sizeof(wm::DevGCol);
+      rc = cuda_check(cudaMalloc(&gcols, bytes), "group columns");
+      if (!rc)
+        rc = cuda_check(cudaMemcpyAsync(gcols, G.gcols.data(), bytes, cudaMemcpyHostToDevice, P->stream),
+                        "group columns");
+    }
     if (!rc)
-      rc = cuda_check(wm::launch_direct_setup(direct_params(P), P->d_gcols, P->d_f64, P->d_direct_cols,
+      rc = cuda_check(cudaMemsetAsync(P->d_direct_seeds, 0, std::max<int64_t>(G.direct_seeds, 1) * sizeof(double2),
+                                      P->stream), "segment seeds");
+    if (!rc)
+      rc = cuda_check(wm::launch_direct_setup(direct_params(P), gcols ? gcols : P->d_gcols, P->d_f64, P->d_direct_cols,
                                               P->d_direct_inj, P->d_direct_seeds, P->stream), "column setup launch");
     if (!rc) rc = cuda_check(cudaStreamSynchronize(P->stream), "column setup");
+    cudaFree(gcols);
   }
   if (!rc && P->split && G.nseeds > 0) {
     wm::FastParams fp = fast_params(P);
