@@ -637,7 +637,7 @@ def run_b200(a):
                         "peak_source": src, "traffic": profile_traffic(dominant),
                         "int8_ops_per_launch": ops, "fp64_equivalent": fp64_view}
         else:
-            roofline = {"bound": "tensor", "kernel": dominant + " (FP64 DMMA)", "achieved": fp64_achieved,
+            roofline = {"bound": "tensor", "kernel": dominant + " (FP64 units)", "achieved": fp64_achieved,
                         "peak": fp64, "unit": "TFLOP/s (fp64)", "frac": fp64_achieved / fp64,
                         "peak_source": fp64_view["peak_source"], "traffic": profile_traffic(dominant),
                         "algorithmic_flops_per_launch": work["legendre_flops"]}
