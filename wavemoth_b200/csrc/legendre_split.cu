@@ -701,8 +701,8 @@ __global__ void __launch_bounds__(kSplitThr, 1) k_a2m_split(SplitParams p) {
 }
 
 // ------------------------------------------------------------------------
-// map2alm residual.  Unit = <= 128 rows of one group, K = all its columns in
-// chunks of 64.  Thread t makes rows 16 (t >> 6) .. + 15 of the unit for
+// map2alm residual.  Unit = <= 128 rows of one group, K = the columns that
+// start before its end, in chunks of 64.  Thread t makes rows 16 (t >> 6) .. + 15 of the unit for
 // chunk column t & 63.
 // ------------------------------------------------------------------------
 __global__ void __launch_bounds__(kSplitThr, 1) k_m2a_split(SplitParams p) {
