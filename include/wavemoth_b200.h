@@ -302,6 +302,12 @@ void wm_host_recurrence_last_row(const double *x2, const double *P0, const doubl
 int wm_host_interp_decomp(double *A, int m, int n, double eps, int *krank, int *perm,
                           double *proj);
 
+/* Whether the FP64 kernels of the interpolation levels hold a depth-1 root of
+   `rows` rows and `skeleton_rows` skeleton rows (both blocks together).  FP64
+   plans leave matrices with larger roots to the kernels for deeper trees,
+   split plans to the split GEMMs whatever their number of maps. */
+int wm_host_level_fits(int64_t rows, int64_t skeleton_rows);
+
 #ifdef __cplusplus
 }
 #endif

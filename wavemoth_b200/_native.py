@@ -33,6 +33,7 @@ HOST_SIGNATURES = {
                                             ctypes.c_int64, c_double_p]),
     "wm_host_interp_decomp": (ctypes.c_int, [c_double_p, ctypes.c_int, ctypes.c_int,
                                              ctypes.c_double, c_int_p, c_int_p, c_double_p]),
+    "wm_host_level_fits": (ctypes.c_int, [ctypes.c_int64, ctypes.c_int64]),
 }
 
 

@@ -479,14 +479,15 @@ int build_direct(DeviceImage &I) {
 }
 
 // The FP64 path of a split image, for its plans of few maps (use_direct):
-// where the plan is large enough to use it, and its tables (at most 8 GiB: an
+// where the plan is large enough to use it, the level kernels hold its roots,
+// and its tables (at most 8 GiB: an
 // nside 1024 plan's are 5) fit beside everything already on the device with a
 // margin of 4 GiB (and under a memory cap).
 constexpr int64_t kDirectMinElems = 4 << 20;
 
 void build_direct_for_split(DeviceImage &I, int64_t plan_bytes) {
   const auto &G = I.prog;
-  if (!I.split || G.rec_elems < kDirectMinElems) return;
+  if (!I.split || G.rec_elems < kDirectMinElems || !wm::level_fits(G.max_root_n, G.max_root_k)) return;
   const int64_t need = G.direct_seeds * (int64_t)sizeof(double2) +
                        (int64_t)G.gcols.size() * (int64_t)(sizeof(wm::DevDirectCol) + wm::kDirectInj * sizeof(double)) +
                        (int64_t)(G.direct_ab.size() + G.direct_scale.size()) * (int64_t)sizeof(double) + (64LL << 20);
@@ -819,7 +820,7 @@ wavemoth_plan make_plan(bool analysis, int Nside, int lmax, int mmax, int nmaps,
       img->prog.shard_m0 = (int32_t)img->m_bounds[part];
       img->prog.shard_m1 = (int32_t)img->m_bounds[part + 1];
     }
-    if (!wm::build_fast_path(img->prog, err)) {
+    if (!wm::build_fast_path(img->prog, (image_flags & WAVEMOTH_PRECISION_SPLIT) != 0, err)) {
       set_error(WAVEMOTH_ERR_RESOURCE, path + ": " + err);
       return nullptr;
     }
@@ -1728,7 +1729,7 @@ int wavemoth_check_resourcefile(char *filename, int Nside, int lmax, int64_t *ou
   wm::HostProgram P;
   if (!wm::compile_resource(file.data(), file.size(), Nside, lmax, lmax, P, err))
     return set_error(WAVEMOTH_ERR_RESOURCE, std::string(filename) + ": " + err);
-  if (!wm::build_fast_path(P, err))
+  if (!wm::build_fast_path(P, false, err))
     return set_error(WAVEMOTH_ERR_RESOURCE, std::string(filename) + ": " + err);
   if (out_stats) {
     out_stats[0] = (int64_t)P.mats.size();

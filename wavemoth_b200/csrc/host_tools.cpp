@@ -21,6 +21,7 @@
 #include <algorithm>
 
 #include "legendre.cuh"
+#include "plan.h"
 
 extern "C" {
 
@@ -144,5 +145,7 @@ void wm_host_recurrence_last_row(const double *x2, const double *P0, const doubl
     out[j] = p;
   }
 }
+
+int wm_host_level_fits(int64_t rows, int64_t skeleton_rows) { return wm::level_fits(rows, skeleton_rows); }
 
 }  // extern "C"

@@ -43,11 +43,6 @@ __device__ __forceinline__ double rec_step(const double *f64, const DevGCol &C, 
   return (x2 + ab[0]) * ab[1] * pc + ab[2] * pp;
 }
 
-// Row stride (doubles) of a staged operand of NT vector tiles: the four rows
-// of a B fragment start in different halves of the 128 bytes of banks.
-template <int NT>
-constexpr int kLevelPitch = NT == 1 ? 8 : 8 * NT + 8;
-
 // D = A x B for rows 8 mt .. + 7 of one interpolation block: A(row, j) =
 // a[row + j lda] (rows beyond `rows` repeat the last one and are not stored),
 // B(j, v) the staged row b(j).  Eight steps of A are in flight at once.
@@ -245,14 +240,8 @@ __global__ void k_seeds(FastParams p) {
 }
 
 template <int NT>
-size_t level_smem(bool alm2map, const FastParams &p) {
-  const size_t rows = p.max_root_n + (alm2map ? p.max_root_k : 0);
-  return rows * kLevelPitch<NT> * sizeof(double) + (size_t)p.max_root_n * 2 * sizeof(int32_t);
-}
-
-template <int NT>
 cudaError_t launch_level_nt(bool alm2map, const FastParams &p, int max_ctas, cudaStream_t st) {
-  const size_t smem = level_smem<NT>(alm2map, p);
+  const size_t smem = (size_t)level_smem_bytes<NT>(alm2map, p.max_root_n, p.max_root_k);
   const int npass = (p.nvecs + 8 * NT - 1) / (8 * NT);
   const int64_t units = (int64_t)p.nroots * npass;
   const int grid = (int)std::min<int64_t>(units, max_ctas > 0 ? max_ctas : INT_MAX);
@@ -271,9 +260,11 @@ cudaError_t launch_level(bool alm2map, const FastParams &p, int max_ctas, cudaSt
   // up to 32 vectors per pass, as few as cover them, and no more than leave
   // room for four CTAs per SM (16 maps at nside 256: 32 vectors per alm2map
   // pass, 82 KB and two CTAs, took 308 us with the residual)
-  constexpr size_t kRoom = 56 * 1024;
-  if (p.nvecs > 16 && level_smem<4>(alm2map, p) <= kRoom) return launch_level_nt<4>(alm2map, p, max_ctas, st);
-  if (p.nvecs > 8 && level_smem<2>(alm2map, p) <= kRoom) return launch_level_nt<2>(alm2map, p, max_ctas, st);
+  constexpr int64_t kRoom = 56 * 1024;
+  if (p.nvecs > 16 && level_smem_bytes<4>(alm2map, p.max_root_n, p.max_root_k) <= kRoom)
+    return launch_level_nt<4>(alm2map, p, max_ctas, st);
+  if (p.nvecs > 8 && level_smem_bytes<2>(alm2map, p.max_root_n, p.max_root_k) <= kRoom)
+    return launch_level_nt<2>(alm2map, p, max_ctas, st);
   return launch_level_nt<1>(alm2map, p, max_ctas, st);
 }
 

@@ -136,6 +136,24 @@ struct DevRootUnit {  // depth-1 level unit: one root's interpolation pair
   int32_t matrix, pair;
 };
 
+// Shared memory of a level kernel (legendre_mma.cu) in a pass of 8 NT vectors,
+// for roots of at most n rows and k skeleton rows: alm2map stages X and the sum
+// over both blocks, map2alm q~, and both the two row permutations.  The row
+// stride (doubles) starts the four rows of a B fragment in different halves of
+// the 128 bytes of banks.
+template <int NT>
+constexpr int kLevelPitch = NT == 1 ? 8 : 8 * NT + 8;
+template <int NT>
+constexpr int64_t level_smem_bytes(bool alm2map, int64_t n, int64_t k) {
+  return (n + (alm2map ? k : 0)) * kLevelPitch<NT> * (int64_t)sizeof(double) + 2 * n * (int64_t)sizeof(int32_t);
+}
+// Whether the FP64 level kernels can run such roots at all, which is up to
+// about 3000 rows: alm2map's narrowest pass, the larger of the two directions',
+// against what a CTA may use (227 KB).  The split path's level GEMMs and the
+// generic kernels take roots of any size.
+constexpr int64_t kMaxCtaSmem = 227 * 1024;
+constexpr bool level_fits(int64_t n, int64_t k) { return level_smem_bytes<1>(true, n, k) <= kMaxCtaSmem; }
+
 constexpr int kSeedRows = 16;   // split path: spacing of the recurrence seeds (P at rows s, s + 1)
 
 // ---- split-precision residual path (sliced int8 operands, tcgen05) ----

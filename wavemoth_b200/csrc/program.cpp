@@ -833,7 +833,7 @@ static void direct_tiles(HostProgram &P, DevGroup &G, int32_t gi) {
   }
 }
 
-bool build_fast_path(HostProgram &P, std::string &err) {
+bool build_fast_path(HostProgram &P, bool split, std::string &err) {
   P.groups.clear();
   P.gcols.clear();
   P.direct_ab.clear();
@@ -874,6 +874,16 @@ bool build_fast_path(HostProgram &P, std::string &err) {
       }
     }
     std::vector<double> ab[2], scale[2];
+    // the level kernels' buffers are sized for the largest root of all matrices
+    int32_t root_k = P.max_root_k, root_n = P.max_root_n;
+    if (ok && M.nlevels == 1) {
+      const DevLevel &L = P.levels[M.level_begin];
+      for (int32_t pi = L.pair_begin; pi < L.pair_end; ++pi) {
+        root_k = std::max(root_k, P.pairs[pi].kT + P.pairs[pi].kB);
+        root_n = std::max(root_n, P.pairs[pi].n);
+      }
+      ok = split || level_fits(root_n, root_k);
+    }
     for (size_t g = 0; ok && g < ranges.size(); ++g)
       ok = direct_coefficients(P, M, (int)g, ranges[g].first, ranges[g].second, ab[g], scale[g]);
     if (!ok) {
@@ -892,9 +902,9 @@ bool build_fast_path(HostProgram &P, std::string &err) {
           return false;
         }
         P.roots.push_back(DevRootUnit{(int32_t)mi, pi});
-        P.max_root_k = std::max(P.max_root_k, pr.kT + pr.kB);
-        P.max_root_n = std::max(P.max_root_n, pr.n);
       }
+      P.max_root_k = root_k;
+      P.max_root_n = root_n;
     }
     for (size_t g = 0; g < ranges.size(); ++g) {
       DevGroup G{};

@@ -87,8 +87,10 @@ inline int64_t q_row(const HostProgram &P, int m, int odd, int64_t ring) {
 enum : int { kStreamResA2M = 0, kStreamResM2A = 1, kStreamLevelA2M = 2, kStreamLevelM2A = 3 };
 
 // Builds the row groups and the tables of both residual paths for matrices
-// of depth 0 and 1.
-bool build_fast_path(HostProgram &P, std::string &err);
+// of depth 0 and 1.  Unless the program is for a split image, matrices whose
+// roots the FP64 level kernels cannot hold (level_fits) are left to the generic
+// kernels.
+bool build_fast_path(HostProgram &P, bool split, std::string &err);
 
 // One serialized butterfly matrix (the per-matrix layout of a rev1 file,
 // starting at its header) compiled without its residual payloads: a single
