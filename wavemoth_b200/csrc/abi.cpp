@@ -1250,6 +1250,14 @@ int finish(wavemoth_plan P, int rc) {
   return rc;
 }
 
+// Whole transforms and hooks on their q need the plan's own q buffer, which a
+// shard does not have (its q buffers are the caller's).
+int whole_plan_check(wavemoth_plan P, const void *a, const void *b) {
+  if (!P || !a || !b) return set_error(WAVEMOTH_ERR_ARG, "NULL plan or buffer");
+  if (P->nparts > 1) return set_error(WAVEMOTH_ERR_ARG, "a shard of a plan runs through the wavemoth_shard_ calls only");
+  return 0;
+}
+
 // The plan's transform on its bound buffers (input -> output), or with
 // adjoint its adjoint (output -> input): for an alm2map plan
 // A^T f = (npix / 4 pi) map2alm(f), for a map2alm plan (4 pi / npix)
@@ -1399,13 +1407,13 @@ int wavemoth_query_resourcefile(char *filename, int *out_Nside, int *out_lmax) {
 
 int wavemoth_execute_alm2map_device(wavemoth_plan plan, const double *alm, double *map,
                                     void *stream) {
-  if (!plan || !alm || !map) return set_error(WAVEMOTH_ERR_ARG, "NULL plan or buffer");
+  if (int rc = whole_plan_check(plan, alm, map)) return rc;
   return finish(plan, run_alm2map(plan, alm, map, (cudaStream_t)stream));
 }
 
 int wavemoth_execute_map2alm_device(wavemoth_plan plan, const double *map, double *alm,
                                     void *stream) {
-  if (!plan || !alm || !map) return set_error(WAVEMOTH_ERR_ARG, "NULL plan or buffer");
+  if (int rc = whole_plan_check(plan, alm, map)) return rc;
   return finish(plan, run_map2alm(plan, map, alm, (cudaStream_t)stream));
 }
 
@@ -1496,12 +1504,12 @@ int wavemoth_shard_map2alm_legendre(wavemoth_plan plan, const double *q_recv, do
 }
 
 int wavemoth_legendre_alm2map_device(wavemoth_plan plan, const double *alm, double *q, void *stream) {
-  if (!plan || !alm || !q || plan->nparts > 1) return set_error(WAVEMOTH_ERR_ARG, "NULL plan or buffer, or a shard");
+  if (int rc = whole_plan_check(plan, alm, q)) return rc;
   return finish(plan, run_legendre(plan, true, alm, nullptr, nullptr, q, (cudaStream_t)stream));
 }
 
 int wavemoth_legendre_map2alm_device(wavemoth_plan plan, const double *q, double *alm, void *stream) {
-  if (!plan || !alm || !q || plan->nparts > 1) return set_error(WAVEMOTH_ERR_ARG, "NULL plan or buffer, or a shard");
+  if (int rc = whole_plan_check(plan, alm, q)) return rc;
   return finish(plan, run_legendre(plan, false, nullptr, alm, q, nullptr, (cudaStream_t)stream));
 }
 
@@ -1526,7 +1534,7 @@ int wavemoth_plan_set_ring_weights(wavemoth_plan plan, const double *weights) {
 }
 
 int wavemoth_alm2map_backward_device(wavemoth_plan plan, const double *grad_map, double *grad_alm, void *stream) {
-  if (!plan || !grad_alm || !grad_map) return set_error(WAVEMOTH_ERR_ARG, "NULL plan or buffer");
+  if (int bad = whole_plan_check(plan, grad_map, grad_alm)) return bad;
   cudaStream_t st = (cudaStream_t)stream;
   const bool fused = weighs_alm(plan);
   int rc = run_map2alm(plan, grad_map, grad_alm, st, 1.0, fused ? AlmOut::kBackward : AlmOut::kWrite);
@@ -1540,7 +1548,8 @@ int wavemoth_alm2map_backward_device(wavemoth_plan plan, const double *grad_map,
 
 int wavemoth_map2alm_iterative_device(wavemoth_plan plan, const double *map, double *alm, int niter,
                                       void *stream) {
-  if (!plan || !alm || !map || niter < 0) return set_error(WAVEMOTH_ERR_ARG, "NULL plan or buffer, or niter < 0");
+  if (int bad = whole_plan_check(plan, map, alm)) return bad;
+  if (niter < 0) return set_error(WAVEMOTH_ERR_ARG, "niter < 0");
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t nmap = plan->npix * plan->nmaps, nalm = plan->nalm * plan->nvecs;
   int rc = 0;
@@ -1567,6 +1576,8 @@ void wavemoth_perform_legendre_transforms(wavemoth_plan plan) {
   int rc = 0;
   if (plan->analysis) {
     rc = set_error(WAVEMOTH_ERR_ARG, "perform_legendre_transforms needs an alm2map plan");
+  } else if (!plan->host_in) {
+    rc = set_error(WAVEMOTH_ERR_ARG, "plan has no bound input buffer");
   } else if (plan->flags & WAVEMOTH_DEVICE_POINTERS) {
     rc = run_legendre(plan, true, plan->host_in, nullptr, nullptr, plan->d_q, plan->stream);
   } else {
@@ -1585,6 +1596,8 @@ void wavemoth_perform_backward_ffts(wavemoth_plan plan) {
   int rc = 0;
   if (plan->analysis) {
     rc = set_error(WAVEMOTH_ERR_ARG, "perform_backward_ffts needs an alm2map plan");
+  } else if (!plan->host_out) {
+    rc = set_error(WAVEMOTH_ERR_ARG, "plan has no bound output buffer");
   } else {
     const bool devptr = (plan->flags & WAVEMOTH_DEVICE_POINTERS) != 0;
     wm::RingParams r = ring_params(plan);
@@ -1603,7 +1616,7 @@ void wavemoth_perform_backward_ffts(wavemoth_plan plan) {
 }
 
 int wavemoth_plan_set_hemisphere_mode(wavemoth_plan plan, int one_side) {
-  if (!plan) return set_error(WAVEMOTH_ERR_ARG, "NULL plan");
+  if (int rc = whole_plan_check(plan, plan, plan)) return rc;
   RingTable RT = ring_table(plan->nside, plan->nmaps, plan->mmax, one_side != 0);
   if (RT.max_cta_cplx > wm::kRingBufferCplx)
     return set_error(WAVEMOTH_ERR_ARG, "ring transforms longer than the CTA buffer");
@@ -1623,7 +1636,7 @@ void wavemoth_disable_phase_shifting(wavemoth_plan plan) {
 }
 
 int wavemoth_get_work(wavemoth_plan plan, double *out) {
-  if (!plan || !out) return set_error(WAVEMOTH_ERR_ARG, "NULL plan or buffer");
+  if (int bad = whole_plan_check(plan, out, out)) return bad;
   const int64_t nrow = 2LL * (plan->mmax + 1) * plan->ni, nv = plan->nvecs;
   std::vector<double> dev((size_t)(nrow * nv));
   int rc = cuda_check(cudaMemcpyAsync(dev.data(), plan->d_q, dev.size() * sizeof(double), cudaMemcpyDeviceToHost,
