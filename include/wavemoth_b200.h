@@ -22,8 +22,8 @@ extern "C" {
 #define WAVEMOTH_PRECISION_SPLIT 0x200   /* residual products of depth-0/1 matrices as sliced int8
                                             tensor-core GEMMs re-summed in FP64 (Ozaki scheme);
                                             the recurrence, seeds and scales stay FP64.  Large
-                                            plans of few maps (up to 8, 14 below nside 512), for
-                                            which that is slower, compute in FP64 throughout */
+                                            plans of few maps, for which that is slower, compute
+                                            in FP64 throughout (wavemoth_plan_route) */
 #define WAVEMOTH_DENSE 0x800            /* no butterfly file: every (m, parity) block as one dense
                                            three-term recurrence over all rings, seeded on the device
                                            (the reference GPU kernel's scheme, wavemoth/cuda/sht.py:20-148);
@@ -33,7 +33,9 @@ extern "C" {
                                             slicing it once per plan into device memory (6 bytes
                                             per element of the residual tiles, about 20 GB at
                                             nside 1024); the plan also falls back to this when
-                                            the device lacks the memory.  Same results. */
+                                            the device lacks the memory.  Same results as the
+                                            GEMMs on stored slices.  Plans of few maps stay on
+                                            the GEMMs too, whose tables this flag saves */
 
 /* status codes */
 #define WAVEMOTH_OK 0
@@ -257,6 +259,20 @@ int wavemoth_plan_set_grid_cap(wavemoth_plan plan, int sms);
    also where its few maps would be computed in FP64.  New; it replaces the reference's abort() on a
    failed check (src/wavemoth_error.h:1-19). */
 int wavemoth_plan_set_wait_limit(wavemoth_plan plan, int64_t polls);
+
+/* The kernels of the plan's Legendre step, decided when the plan is made (and
+   by a wait limit).  FP64 plans: WAVEMOTH_ROUTE_FP64.  Split plans: the same for
+   up to 8 maps, or 14 where the file's recurrence and interpolation elements
+   (wavemoth_plan_work, out[5] + out[4]) are 80 million at most, on files of
+   2^22 recurrence elements and more whose roots fit (wm_host_level_fits), if
+   the device had room for the FP64 tables (8 GiB at most) with 4 GiB to spare
+   when the plan was made; else the split GEMMs, on slices of P made once per
+   image or, without room for them or with WAVEMOTH_SPLIT_GENERATE, generated by
+   every call (equal results).  -1 for a NULL plan.  New. */
+#define WAVEMOTH_ROUTE_FP64 0
+#define WAVEMOTH_ROUTE_GEMM 1
+#define WAVEMOTH_ROUTE_GEMM_GENERATE 2
+int wavemoth_plan_route(wavemoth_plan plan);
 
 /* Per-kernel device timing of a plan, from CUDA events recorded on the
    launching stream.  mode 1: reset and enable, 0: reset and disable,

@@ -45,6 +45,7 @@ SIGNATURES = {
     "wavemoth_plan_image_bytes": (ctypes.c_int64, [_vp]),
     "wavemoth_set_device_memory_cap": (None, [ctypes.c_int64]),
     "wavemoth_plan_set_wait_limit": (ctypes.c_int, [_vp, ctypes.c_int64]),
+    "wavemoth_plan_route": (ctypes.c_int, [_vp]),
     "wavemoth_execute_adjoint": (None, [_vp]),
     "wavemoth_plan_set_ring_weights": (ctypes.c_int, [_vp, _dp]),
     "wavemoth_legendre_alm2map_device": (ctypes.c_int, [_vp, _vp, _vp, _vp]),

@@ -56,13 +56,22 @@ struct DeviceArena {
     *out = (T *)p;
     return 0;
   }
+  // Takes over the allocations of another arena.
+  void adopt(DeviceArena &other) {
+    ptrs.insert(ptrs.end(), other.ptrs.begin(), other.ptrs.end());
+    bytes += other.bytes;
+    other.ptrs.clear();
+    other.bytes = 0;
+  }
 };
 
 }  // namespace
 
 // Device data of a compiled plan file that does not depend on the number of
-// maps: the butterfly program, the tensor-core and split tables, the ring
-// tables, the sliced P and W.  Read-only once built.
+// maps: the butterfly program, the tables of the FP64 and of the split path,
+// the ring tables, the sliced P and W.  Read-only once built; what only some
+// plans of a split image read (the FP64 tables, the sliced P) is added when the
+// first of them is made, and plans see what there was when they were made.
 struct ImageRefs {
   wm::DevMatrix *d_mats = nullptr;
   wm::DevDBlock *d_dblocks = nullptr;
@@ -362,7 +371,7 @@ wm::FastParams fast_params(wavemoth_plan P) {
   f.gcols = P->d_gcols;
   f.roots = P->d_roots;
   f.ngroups = (int32_t)G.groups.size();
-  f.ngcols = (int64_t)G.gcols.size();
+  f.ngcols = G.ngcols;
   f.nroots = (int32_t)G.roots.size();
   f.max_root_k = G.max_root_k;
   f.max_root_n = G.max_root_n;
@@ -386,7 +395,7 @@ wm::DirectParams direct_params(wavemoth_plan P) {
   d.tiles_b = P->d_direct_b;
   d.ntiles_b = P->ndirect_b;
   d.ngroups = (int32_t)P->img->prog.groups.size();
-  d.ngcols = (int64_t)P->img->prog.gcols.size();
+  d.ngcols = P->img->prog.ngcols;
   d.lmax = P->lmax;
   d.nvecs = P->nvecs;
   d.q_mstride = P->nvecs;
@@ -406,7 +415,7 @@ wm::SplitParams split_params(wavemoth_plan P) {
   s.tiles_a = P->d_stiles_a;
   s.tiles_b = P->d_stiles_b;
   s.ngroups = (int32_t)G.groups.size();
-  s.ngcols = (int64_t)G.gcols.size();
+  s.ngcols = G.ngcols;
   s.ntiles_a = (int32_t)G.stiles_a.size();
   s.ntiles_b = (int32_t)G.stiles_b.size();
   s.seeds = P->d_seeds;
@@ -437,6 +446,33 @@ wm::SplitParams split_params(wavemoth_plan P) {
   return s;
 }
 
+// Whether a split plan's number of maps puts its Legendre step on the FP64
+// units, on images large enough (kDirectMinElems) whose roots the level kernels
+// hold.  The split GEMMs stream six bytes of sliced P per element whatever the
+// number of maps, the FP64 kernels do two operations and one per vector.
+// Measured, alm2map + map2alm, FP64 / split, us: nside 128, lmax 256: 3 maps 43
+// / 130, 16 maps 106 / 138; nside 256, lmax 512: 8 maps 284 / 485, 16 maps 500 /
+// 507; nside 512, lmax 1024: 8 maps 1501 / 2261, 16 maps 2861 / 2330; nside 1024,
+// lmax 1500: 3 maps 2841 / 7254, 8 maps 5474 / 7532, 16 maps 10660 / 7838.  Plans
+// that are to generate P rather than hold it would hold the FP64 tables instead,
+// and keep the GEMMs.
+constexpr int64_t kDirectMinElems = 4 << 20;
+
+bool prefers_direct(wavemoth_plan P) {
+  const auto &G = P->img->prog;
+  if ((P->flags & WAVEMOTH_SPLIT_GENERATE) || G.rec_elems < kDirectMinElems ||
+      !wm::level_fits(G.max_root_n, G.max_root_k))
+    return false;
+  return P->nvecs <= (G.rec_elems + G.interp_elems <= 80000000 ? 28 : 16);
+}
+
+// Whether a plan's Legendre step runs on the FP64 units: always without split
+// precision, and with it where that is preferred and the image has the tables.
+// A plan with a wait limit set keeps the kernels whose waits it bounds.
+bool use_direct(wavemoth_plan P) {
+  return !P->split || (P->direct && P->wait_limit == 0 && prefers_direct(P));
+}
+
 // Images of compiled plan files, shared by the plans that use the same file
 // (path, size, modification time), lmax, mmax and precision flags; an image
 // lives as long as one of its plans.  Plan creation is serialised.
@@ -454,11 +490,9 @@ struct ImageKey {
 std::mutex g_image_mutex;
 std::map<ImageKey, std::weak_ptr<DeviceImage>> g_images;
 
-// Tables of the FP64 residual path (filled by init_image).
-int build_direct(DeviceImage &I) {
-  auto &G = I.prog;
-  DeviceArena &A = I.arena;
-  const size_t nc = G.gcols.size();
+// Tables of the FP64 residual path, allocated in A (setup_direct fills them).
+int build_direct(ImageRefs &I, const wm::HostProgram &G, DeviceArena &A) {
+  const size_t nc = (size_t)G.ngcols;
   int rc = 0;
   for (int w = 0; w < 2; ++w) {
     wm::DevDirectTileA *tiles = nullptr;
@@ -476,25 +510,6 @@ int build_direct(DeviceImage &I) {
   rc = rc ? rc : A.alloc(&I.d_direct_seeds, (size_t)G.direct_seeds, "segment seeds");
   I.direct = rc == 0;
   return rc;
-}
-
-// The FP64 path of a split image, for its plans of few maps (use_direct):
-// where the plan is large enough to use it, the level kernels hold its roots,
-// and its tables (at most 8 GiB: an
-// nside 1024 plan's are 5) fit beside everything already on the device with a
-// margin of 4 GiB (and under a memory cap).
-constexpr int64_t kDirectMinElems = 4 << 20;
-
-void build_direct_for_split(DeviceImage &I, int64_t plan_bytes) {
-  const auto &G = I.prog;
-  if (!I.split || G.rec_elems < kDirectMinElems || !wm::level_fits(G.max_root_n, G.max_root_k)) return;
-  const int64_t need = G.direct_seeds * (int64_t)sizeof(double2) +
-                       (int64_t)G.gcols.size() * (int64_t)(sizeof(wm::DevDirectCol) + wm::kDirectInj * sizeof(double)) +
-                       (int64_t)(G.direct_ab.size() + G.direct_scale.size()) * (int64_t)sizeof(double) + (64LL << 20);
-  size_t fr = 0, tot = 0;
-  if (need > (8LL << 30) || cudaMemGetInfo(&fr, &tot) != cudaSuccess || (int64_t)fr < need + (4LL << 30)) return;
-  if (g_device_cap > 0 && I.arena.bytes + plan_bytes + need > g_device_cap) return;
-  build_direct(I);
 }
 
 // Uploads the map-count independent tables of `img` (whose program is
@@ -533,7 +548,7 @@ int build_image(DeviceImage &I, int nside, int mmax, unsigned flags) {
   if (flags & WAVEMOTH_PRECISION_SPLIT) rc = rc ? rc : upload(A, &I.d_gcols, G.gcols, "group columns");
   rc = rc ? rc : upload(A, &I.d_roots, G.roots, "roots");
   I.split = (flags & WAVEMOTH_PRECISION_SPLIT) != 0;
-  if (!I.split) rc = rc ? rc : build_direct(I);
+  if (!I.split) rc = rc ? rc : build_direct(I, G, A);
   if (I.split) rc = rc ? rc : A.alloc(&I.d_seeds, (size_t)std::max<int64_t>(G.nseeds, 1), "recurrence seeds");
   I.program_bytes = A.bytes;
   {
@@ -574,49 +589,131 @@ int build_image(DeviceImage &I, int nside, int mmax, unsigned flags) {
   return rc;
 }
 
-// The residual P slices of a split image, when they fit beside everything
-// already on the device with a margin of 4 GiB (and under a memory cap).
-void alloc_residual_slices(DeviceImage &I, int64_t plan_bytes, unsigned flags) {
-  const auto &G = I.prog;
-  if (!I.split || (flags & WAVEMOTH_SPLIT_GENERATE) || G.stream_res_blocks <= 0) return;
-  const int64_t need = G.stream_res_blocks * (int64_t)wm::kSplitBlock;
+// Whether `need` more bytes fit beside everything already on the device with a
+// margin of 4 GiB, and under a memory cap.
+bool device_room(wavemoth_plan P, int64_t need) {
   size_t fr = 0, tot = 0;
-  bool fits = cudaMemGetInfo(&fr, &tot) == cudaSuccess && (int64_t)fr > need + (4LL << 30);
-  if (g_device_cap > 0 && I.arena.bytes + plan_bytes + need > g_device_cap) fits = false;
-  if (fits && I.arena.alloc(&I.d_res_a, (size_t)need, "sliced residual P") == 0) I.res_a_bytes = need;
-  else I.d_res_a = nullptr;
+  if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return (int64_t)fr > need + (4LL << 30) &&
+         !(g_device_cap > 0 && P->img->arena.bytes + P->arena.bytes + need > g_device_cap);
+}
+
+void free_host_direct(wm::HostProgram &G) {
+  G.direct_ab.clear(); G.direct_ab.shrink_to_fit();
+  G.direct_scale.clear(); G.direct_scale.shrink_to_fit();
+  G.direct_tile_seeds.clear(); G.direct_tile_seeds.shrink_to_fit();
+}
+
+// Fills the plan's FP64 tables from its group columns.
+int setup_direct(wavemoth_plan P) {
+  auto &G = P->img->prog;
+  if (!G.ngcols) return 0;
+  // the uploads went through the default stream, which the plan's does not wait for
+  int rc = cuda_check(cudaStreamSynchronize(0), "image upload");
+  wm::DevGCol *gcols = nullptr;
+  if (!rc && !P->d_gcols) {
+    const size_t bytes = G.gcols.size() * sizeof(wm::DevGCol);
+    rc = cuda_check(cudaMalloc(&gcols, bytes), "group columns");
+    if (!rc)
+      rc = cuda_check(cudaMemcpyAsync(gcols, G.gcols.data(), bytes, cudaMemcpyHostToDevice, P->stream),
+                      "group columns");
+  }
+  if (!rc)
+    rc = cuda_check(cudaMemsetAsync(P->d_direct_seeds, 0, std::max<int64_t>(G.direct_seeds, 1) * sizeof(double2),
+                                    P->stream), "segment seeds");
+  if (!rc)
+    rc = cuda_check(wm::launch_direct_setup(direct_params(P), gcols ? gcols : P->d_gcols, P->d_f64, P->d_direct_cols,
+                                            P->d_direct_inj, P->d_direct_seeds, P->stream), "column setup launch");
+  if (!rc) rc = cuda_check(cudaStreamSynchronize(P->stream), "column setup");
+  cudaFree(gcols);
+  return rc;
+}
+
+// The FP64 tables of a split image, at most 8 GiB (an nside 1024 plan's are 5)
+// and where they fit; without them the plan keeps to the split GEMMs.
+int provide_direct(wavemoth_plan P) {
+  DeviceImage &I = *P->img;
+  auto &G = I.prog;
+  if (!I.direct) {
+    const int64_t need = G.direct_seeds * (int64_t)sizeof(double2) +
+                         G.ngcols * (int64_t)(sizeof(wm::DevDirectCol) + wm::kDirectInj * sizeof(double)) +
+                         (int64_t)(G.direct_ab.size() + G.direct_scale.size()) * (int64_t)sizeof(double) + (64LL << 20);
+    if (need > (8LL << 30) || !device_room(P, need)) return 0;
+    DeviceArena A;
+    A.base = I.arena.bytes + P->arena.bytes;
+    ImageRefs R = I;
+    if (build_direct(R, G, A)) {
+      cudaGetLastError();  // another process took the memory
+      return 0;
+    }
+    static_cast<ImageRefs &>(*P) = R;
+    if (int rc = setup_direct(P)) return rc;
+    static_cast<ImageRefs &>(I) = R;
+    I.arena.adopt(A);
+    free_host_direct(G);
+  }
+  static_cast<ImageRefs &>(*P) = I;
+  return 0;
+}
+
+// The sliced residual P of a split image, where it fits; without it the GEMM
+// kernels generate P at every call.
+int provide_slices(wavemoth_plan P) {
+  DeviceImage &I = *P->img;
+  const auto &G = I.prog;
+  if ((P->flags & WAVEMOTH_SPLIT_GENERATE) || G.stream_res_blocks <= 0) return 0;
+  if (!I.d_res_a) {
+    const int64_t need = G.stream_res_blocks * (int64_t)wm::kSplitBlock;
+    if (!device_room(P, need)) return 0;
+    DeviceArena A;
+    A.base = I.arena.bytes + P->arena.bytes;
+    if (A.alloc(&P->d_res_a, (size_t)need, "sliced residual P")) {
+      cudaGetLastError();
+      return 0;
+    }
+    const wm::SplitParams sp = split_params(P);
+    int rc = cuda_check(wm::launch_residual_slices(sp, stream_launch(P, wm::kStreamResA2M),
+                                                   stream_launch(P, wm::kStreamResM2A), P->stream),
+                        "residual slice launch");
+    if (!rc) rc = cuda_check(cudaStreamSynchronize(P->stream), "residual slices");
+    if (rc) {
+      P->d_res_a = nullptr;
+      return rc;
+    }
+    I.d_res_a = P->d_res_a;
+    I.res_a_bytes = need;
+    I.arena.adopt(A);
+  }
+  P->d_res_a = I.d_res_a;
+  P->res_a_bytes = I.res_a_bytes;
+  return 0;
+}
+
+// Makes a split image hold what this plan's residual products read and earlier
+// plans did not.  An nside 1024 image then has tens of GB of sliced P only if a
+// plan of many maps reads it, and 5 GB of FP64 tables only if one of few does.
+int provide_residual(wavemoth_plan P) {
+  if (!P->split) return 0;
+  if (prefers_direct(P))
+    if (int rc = provide_direct(P)) return rc;
+  return use_direct(P) ? 0 : provide_slices(P);
 }
 
 // Plan-time kernels of a new image, run through its first plan: ring
-// tables, recurrence seeds, split scales and slices.
+// tables, FP64 tables, recurrence seeds, split scales and level slices.
 int init_image(wavemoth_plan P) {
   auto &G = P->img->prog;
-  // the uploads went through the default stream, which the plan's does not wait for
-  int rc = cuda_check(cudaStreamSynchronize(0), "image upload");
+  int rc = cuda_check(cudaStreamSynchronize(0), "image upload");  // as in setup_direct
   if (!rc) {
     wm::RingParams rp = ring_params(P);
     rc = cuda_check(wm::launch_ring_setup(rp, P->d_twiddles, P->max_bluestein ? P->d_filters : nullptr,
                                           P->d_ring_aux, P->d_phases, P->stream), "ring setup launch");
     if (!rc) rc = cuda_check(cudaStreamSynchronize(P->stream), "ring setup");
   }
-  if (!rc && P->direct && !G.gcols.empty()) {
-    wm::DevGCol *gcols = nullptr;
-    if (!P->d_gcols) {
-      const size_t bytes = G.gcols.size() * sizeof(wm::DevGCol);
-      rc = cuda_check(cudaMalloc(&gcols, bytes), "group columns");
-      if (!rc)
-        rc = cuda_check(cudaMemcpyAsync(gcols, G.gcols.data(), bytes, cudaMemcpyHostToDevice, P->stream),
-                        "group columns");
-    }
-    if (!rc)
-      rc = cuda_check(cudaMemsetAsync(P->d_direct_seeds, 0, std::max<int64_t>(G.direct_seeds, 1) * sizeof(double2),
-                                      P->stream), "segment seeds");
-    if (!rc)
-      rc = cuda_check(wm::launch_direct_setup(direct_params(P), gcols ? gcols : P->d_gcols, P->d_f64, P->d_direct_cols,
-                                              P->d_direct_inj, P->d_direct_seeds, P->stream), "column setup launch");
-    if (!rc) rc = cuda_check(cudaStreamSynchronize(P->stream), "column setup");
-    cudaFree(gcols);
-  }
+  if (!rc && !P->split) rc = setup_direct(P);
   if (!rc && P->split && G.nseeds > 0) {
     wm::FastParams fp = fast_params(P);
     fp.seeds_out = P->d_seeds;
@@ -636,10 +733,6 @@ int init_image(wavemoth_plan P) {
       sp.rowmax = rowmax;
       rc = cuda_check(wm::launch_split_scales(sp, P->stream), "split scale launch");
       if (!rc) rc = cuda_check(wm::launch_level_slices(sp, P->stream), "level slice launch");
-      if (!rc && P->d_res_a)
-        rc = cuda_check(wm::launch_residual_slices(sp, stream_launch(P, wm::kStreamResA2M),
-                                                   stream_launch(P, wm::kStreamResM2A), P->stream),
-                        "residual slice launch");
       if (!rc) rc = cuda_check(cudaStreamSynchronize(P->stream), "split scales");
     }
     cudaFree(colmax);
@@ -653,9 +746,7 @@ int init_image(wavemoth_plan P) {
     G.f64.clear(); G.f64.shrink_to_fit();
     G.i32.clear(); G.i32.shrink_to_fit();
     G.gcols.clear(); G.gcols.shrink_to_fit();
-    G.direct_ab.clear(); G.direct_ab.shrink_to_fit();
-    G.direct_scale.clear(); G.direct_scale.shrink_to_fit();
-    G.direct_tile_seeds.clear(); G.direct_tile_seeds.shrink_to_fit();
+    if (!P->split) free_host_direct(G);
   }
   return rc;
 }
@@ -918,16 +1009,13 @@ wavemoth_plan make_plan(bool analysis, int Nside, int lmax, int mmax, int nmaps,
     rc = rc ? rc : A.alloc(&P->d_alm, (size_t)P->nalm * P->nvecs, "alm buffer");
     rc = rc ? rc : A.alloc(&P->d_map, (size_t)P->npix * nmaps, "map buffer");
   }
-  if (!rc && fresh) {
-    alloc_residual_slices(*img, A.bytes, flags);
-    build_direct_for_split(*img, A.bytes);
-    A.base = img->arena.bytes;
-  }
   static_cast<ImageRefs &>(*P) = static_cast<const ImageRefs &>(*img);
   rc = rc ? rc : cuda_check(cudaStreamCreateWithFlags(&P->stream, cudaStreamNonBlocking),
                             "cudaStreamCreate");
   if (!rc) rc = cuda_check(cudaMemsetAsync(P->d_status, 0, sizeof(int32_t), P->stream), "status reset");
   if (!rc && fresh) rc = init_image(P);
+  if (!rc) rc = provide_residual(P);
+  A.base = img->arena.bytes;
   if (!rc) rc = cuda_check(cudaStreamSynchronize(P->stream), "plan setup");
   if (!rc) rc = prepare_noalloc();
   if (rc) {
@@ -1110,22 +1198,6 @@ int run_split(wavemoth_plan P, bool alm2map, const double *alm_in, double *alm_o
 // What map2alm does with the alm it computes: writes it, adds it, or writes it
 // as the gradient of a real map (rows of m > 0 twice, Im a_l0 zero).
 enum class AlmOut { kWrite, kAdd, kBackward };
-
-// Whether a plan's Legendre step runs on the FP64 units: always without split
-// precision, and with it where that is faster.  The split GEMMs stream six
-// bytes of sliced P per element whatever the number of maps, the FP64 kernels
-// do two operations and one per vector.  Measured, alm2map + map2alm, FP64 /
-// split, us: nside 128, lmax 256: 3 maps 43 / 130, 16 maps 106 / 138; nside
-// 256, lmax 512: 8 maps 284 / 485, 16 maps 500 / 507; nside 512, lmax 1024:
-// 8 maps 1501 / 2261, 16 maps 2861 / 2330; nside 1024, lmax 1500: 3 maps 2841
-// / 7254, 8 maps 5474 / 7532, 16 maps 10660 / 7838.  A plan with a wait limit
-// set keeps the kernels whose waits it bounds.
-bool use_direct(wavemoth_plan P) {
-  if (!P->split) return true;
-  if (!P->direct || P->wait_limit > 0) return false;
-  const auto &G = P->img->prog;
-  return P->nvecs <= (G.rec_elems + G.interp_elems <= 80000000 ? 28 : 16);
-}
 
 // FP64 path: residual products, and the interpolation levels of depth-1
 // matrices after (alm2map) or before them (map2alm).
@@ -1671,7 +1743,21 @@ int wavemoth_plan_set_grid_cap(wavemoth_plan plan, int sms) {
 int wavemoth_plan_set_wait_limit(wavemoth_plan plan, int64_t polls) {
   if (!plan || polls < 0) return set_error(WAVEMOTH_ERR_ARG, "wavemoth_plan_set_wait_limit: bad argument");
   plan->wait_limit = polls;
-  return 0;
+  if (!plan->split || use_direct(plan) || plan->d_res_a) return 0;
+  // a plan of few maps that is now to run the GEMMs.  Allocating and running on
+  // the plan's own stream disturbs no capture, which the driver is told
+  std::lock_guard<std::mutex> lock(g_image_mutex);
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  const int rc = provide_slices(plan);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  plan->arena.base = plan->img->arena.bytes;
+  return rc;
+}
+
+int wavemoth_plan_route(wavemoth_plan plan) {
+  if (!plan) return -1;
+  return use_direct(plan) ? WAVEMOTH_ROUTE_FP64 : plan->d_res_a ? WAVEMOTH_ROUTE_GEMM : WAVEMOTH_ROUTE_GEMM_GENERATE;
 }
 
 int wavemoth_plan_timing(wavemoth_plan plan, int mode, double *out) {

@@ -956,6 +956,7 @@ bool build_fast_path(HostProgram &P, bool split, std::string &err) {
       P.groups.push_back(G);
     }
   }
+  P.ngcols = (int64_t)P.gcols.size();
   auto rows_left = [&](const DevDirectTileA &t) { return P.groups[t.group].nrows - t.kstart; };
   for (auto &t : P.direct_a)
     std::stable_sort(t.begin(), t.end(), [&](const DevDirectTileA &a, const DevDirectTileA &b) {

@@ -24,7 +24,8 @@ struct HostProgram {
   std::vector<int64_t> element_count;   // header element_count per (2m + odd)
   // row groups and their tables (see plan.h)
   std::vector<DevGroup> groups;
-  std::vector<DevGCol> gcols;
+  std::vector<DevGCol> gcols;           // freed once the image is made
+  int64_t ngcols = 0;                   // their number
   std::vector<double> direct_ab;        // FP64 path: (A, B) per group row
   std::vector<double> direct_scale;     // and s
   std::vector<DevDirectTileA> direct_a[2];              // alm2map units (narrow, wide), largest first

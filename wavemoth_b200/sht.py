@@ -18,8 +18,9 @@ class Transform:
     """Both directions share one device plan (the compiled butterfly program
     serves A^T for alm2map and A for map2alm).  precision='split' runs the
     residual and level products as sliced int8 tensor-core GEMMs re-summed in
-    FP64 ('split-generate': the residual P regenerated at every call instead
-    of held sliced in device memory)."""
+    FP64, or for few maps, where those are slower, on the FP64 kernels (see
+    `route`); 'split-generate' always runs the GEMMs, with the residual P
+    regenerated at every call instead of held sliced in device memory."""
 
     def __init__(self, resource_file, nside, lmax, nmaps=1, precision="double", dense=False):
         """dense=True: no butterfly file (resource_file may be None); every
@@ -125,6 +126,12 @@ class Transform:
     @property
     def plan_handle(self):
         return self._plan
+
+    @property
+    def route(self):
+        """Kernels of the Legendre step (wavemoth_plan_route): "fp64", "gemm"
+        (split products on stored slices) or "gemm-generate"."""
+        return ("fp64", "gemm", "gemm-generate")[_native.lib().wavemoth_plan_route(self._plan)]
 
     def timing(self, mode):
         """Per-kernel event timing: mode 1 enable/reset, 0 disable, 2 read
