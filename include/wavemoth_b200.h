@@ -220,8 +220,9 @@ int wavemoth_plan_set_ring_weights(wavemoth_plan plan, const double *weights);
 /* Gradient of a real loss with respect to the alm of alm2map, from its
    gradient with respect to the map (device pointers, enqueued on `stream`):
    (npix / 4 pi) c_m map2alm(grad_map), c_0 = 1, c_m = 2, and Im a_l0 = 0,
-   re/im of every (l, m >= 0) entry being independent variables.  Ring
-   weights, if set, apply as in map2alm. */
+   re/im of every (l, m >= 0) entry being independent variables.  map2alm here
+   is the unweighted one: alm2map has no ring weights, so its gradient does not
+   depend on those set on the plan. */
 int wavemoth_alm2map_backward_device(wavemoth_plan plan, const double *grad_map, double *grad_alm, void *stream);
 
 /* map2alm refined by niter Jacobi iterations, a_{k+1} = a_k +
@@ -234,7 +235,7 @@ int wavemoth_map2alm_iterative_device(wavemoth_plan plan, const double *map, dou
 
 /* The adjoint of the plan's transform on its bound buffers: reads the
    output buffer, writes the input buffer.  alm2map plan: alm = (Npix / 4 pi)
-   map2alm(map); map2alm plan: map = (4 pi / Npix) alm2map(alm) -- the
+   map2alm(map), without ring weights; map2alm plan: map = (4 pi / Npix) alm2map(alm) -- the
    adjoints with respect to the real inner product on maps and
    <a, b> = sum_lm c_m Re(a_lm conj b_lm), c_0 = 1, c_m = 2, on alm.  Status
    through wavemoth_plan_status.  New: the reference has no analysis

@@ -1288,16 +1288,20 @@ int run_alm2map(wavemoth_plan P, const double *alm, double *map, cudaStream_t st
   return rc;
 }
 
-// scale multiplies q~ (4 pi / npix for map2alm; 1 for the adjoint of alm2map)
-int run_map2alm(wavemoth_plan P, const double *map, double *alm, cudaStream_t st, double scale = -1.0,
+// map2alm, or (adjoint) (npix / 4 pi) times it without the ring weights, the
+// adjoint of alm2map
+int run_map2alm(wavemoth_plan P, const double *map, double *alm, cudaStream_t st, bool adjoint = false,
                 AlmOut how = AlmOut::kWrite) {
   wm::RingParams r = ring_params(P);
+  if (adjoint) {
+    r.scale = 1.0;
+    r.ring_weights = nullptr;
+  }
   r.map_in = map;
   r.q_out = P->d_q;
   // q~ is consumed by this plan's Legendre step, which weighs the rows above
   // each ring's m limit by Legendre values below 1e-30: written as zeros
   r.ring_mend = P->d_ring_mend;
-  if (scale >= 0.0) r.scale = scale;
   int sp = span_begin(P, 3, st);
   int rc0 = cuda_check(wm::launch_ring_analysis(r, st), "ring analysis launch");
   P->kernel_launches += r.ntasks > 0;
@@ -1362,7 +1366,7 @@ int host_execute(wavemoth_plan P, bool adjoint = false) {
     if (!devptr)
       rc = cuda_check(cudaMemcpyAsync(P->d_map, map_host, map_bytes, cudaMemcpyHostToDevice, st),
                       "map upload");
-    rc = rc ? rc : run_map2alm(P, map, alm, st, adjoint ? 1.0 : -1.0);
+    rc = rc ? rc : run_map2alm(P, map, alm, st, adjoint);
     if (!devptr && !rc)
       rc = cuda_check(cudaMemcpyAsync(alm_host, P->d_alm, alm_bytes, cudaMemcpyDeviceToHost, st),
                       "alm download");
@@ -1609,7 +1613,7 @@ int wavemoth_alm2map_backward_device(wavemoth_plan plan, const double *grad_map,
   if (int bad = whole_plan_check(plan, grad_map, grad_alm)) return bad;
   cudaStream_t st = (cudaStream_t)stream;
   const bool fused = weighs_alm(plan);
-  int rc = run_map2alm(plan, grad_map, grad_alm, st, 1.0, fused ? AlmOut::kBackward : AlmOut::kWrite);
+  int rc = run_map2alm(plan, grad_map, grad_alm, st, true, fused ? AlmOut::kBackward : AlmOut::kWrite);
   if (!rc && !fused) {
     rc = cuda_check(wm::launch_backward_weights(grad_alm, plan->lmax + 1, plan->nalm, plan->nvecs, st),
                     "backward weights");
@@ -1634,7 +1638,7 @@ int wavemoth_map2alm_iterative_device(wavemoth_plan plan, const double *map, dou
   for (int it = 0; it < niter && !rc; ++it) {
     // a += map2alm(f - alm2map(a))
     rc = run_alm2map(plan, alm, plan->d_iter_map, st, 1.0, map);
-    if (!rc) rc = run_map2alm(plan, plan->d_iter_map, add ? alm : plan->d_iter_alm, st, -1.0,
+    if (!rc) rc = run_map2alm(plan, plan->d_iter_map, add ? alm : plan->d_iter_alm, st, false,
                               add ? AlmOut::kAdd : AlmOut::kWrite);
     if (rc || add) continue;
     rc = cuda_check(wm::launch_accumulate(plan->d_iter_alm, alm, nalm, st), "accumulate");

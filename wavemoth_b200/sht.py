@@ -88,7 +88,8 @@ class Transform:
     def alm2map_backward(self, grad_map, out=None):
         """Gradient of a loss with respect to the alm of alm2map, from its
         gradient with respect to the map: (npix / 4 pi) c_m map2alm(grad_map),
-        c_0 = 1, c_m = 2, with Im a_l0 zero (re/im as independent variables)."""
+        c_0 = 1, c_m = 2, with Im a_l0 zero (re/im as independent variables).
+        Ring weights do not enter: alm2map has none."""
         grad_map = self._check_map(grad_map)
         if out is None:
             out = torch.empty((self.nalm, self.nmaps), dtype=torch.complex128, device=grad_map.device)
