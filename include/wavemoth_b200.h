@@ -235,8 +235,9 @@ int wavemoth_map2alm_iterative_device(wavemoth_plan plan, const double *map, dou
 
 /* The adjoint of the plan's transform on its bound buffers: reads the
    output buffer, writes the input buffer.  alm2map plan: alm = (Npix / 4 pi)
-   map2alm(map), without ring weights; map2alm plan: map = (4 pi / Npix) alm2map(alm) -- the
-   adjoints with respect to the real inner product on maps and
+   map2alm(map), without ring weights; map2alm plan: map = (4 pi / Npix)
+   alm2map(alm), times the ring weights if set -- the adjoints with respect
+   to the real inner product on maps and
    <a, b> = sum_lm c_m Re(a_lm conj b_lm), c_0 = 1, c_m = 2, on alm.  Status
    through wavemoth_plan_status.  New: the reference has no analysis
    direction (src/wavemoth.c:1271-1283 is synthesis only). */

@@ -14,7 +14,9 @@ the alm: Transform.alm2map_backward; no Legendre values are stored: the backward
 pass regenerates them with the same recurrence as the forward pass):
 
     alm2map backward:  grad_alm = (Npix / 4 pi) c_m map2alm(grad_map)
-    map2alm backward:  grad_map = (4 pi / Npix) alm2map(grad_alm / c_m)
+    map2alm backward:  grad_map = (4 pi / Npix) w_ring alm2map(grad_alm / c_m)
+
+with w_ring the ring weights set on the Transform at the forward call (1 without).
 
 For complex tensors torch expects grad = dL/dRe + i dL/dIm, which is the
 componentwise real gradient above.  Im a_l0 gets a zero gradient (the forward
@@ -23,8 +25,10 @@ transform ignores it).  The forward definitions follow src/wavemoth.c:1011-1191
 """
 import math
 
+import numpy as np
 import torch
 
+from .healpix import get_ring_pixel_counts
 from .sht import Transform
 
 
@@ -33,6 +37,13 @@ def _m_weights(lmax, device):
     w = torch.full(((lmax + 1) * (lmax + 2) // 2,), 2.0, dtype=torch.float64, device=device)
     w[: lmax + 1] = 1.0
     return w
+
+
+def _pixel_weights(nside, ring_weights, device):
+    """(npix, 1) weight of every pixel: that of its ring's pair (equator first)."""
+    pair = np.abs(np.arange(4 * nside - 1) - (2 * nside - 1))
+    w = torch.from_numpy(np.repeat(ring_weights[pair], get_ring_pixel_counts(nside)))
+    return w.to(device)[:, None]
 
 
 class _Alm2Map(torch.autograd.Function):
@@ -50,6 +61,7 @@ class _Map2Alm(torch.autograd.Function):
     @staticmethod
     def forward(ctx, maps, transform):
         ctx.transform = transform
+        ctx.ring_weights = getattr(transform, "ring_weights", None)
         return transform.map2alm(maps)
 
     @staticmethod
@@ -59,8 +71,10 @@ class _Map2Alm(torch.autograd.Function):
         g = (grad_alm / w[:, None]).contiguous()
         # Im of m = 0 rows is not an output of map2alm: drop its cotangent
         g[: T.lmax + 1] = g[: T.lmax + 1].real.to(torch.complex128)
-        out = T.alm2map(g)
-        return out * (4.0 * math.pi / T.npix), None
+        out = T.alm2map(g) * (4.0 * math.pi / T.npix)
+        if ctx.ring_weights is not None:
+            out = out * _pixel_weights(T.nside, ctx.ring_weights, out.device)
+        return out, None
 
 
 def alm2map(alm, transform):

@@ -1337,7 +1337,7 @@ int whole_plan_check(wavemoth_plan P, const void *a, const void *b) {
 // The plan's transform on its bound buffers (input -> output), or with
 // adjoint its adjoint (output -> input): for an alm2map plan
 // A^T f = (npix / 4 pi) map2alm(f), for a map2alm plan (4 pi / npix)
-// alm2map(a), both with respect to the real inner product on maps and
+// alm2map(a) times the ring weights, both with respect to the real inner product on maps and
 // <a, b> = sum_lm c_m Re(a_lm conj b_lm) (c_0 = 1, c_m = 2) on alm.
 int host_execute(wavemoth_plan P, bool adjoint = false) {
   cudaStream_t st = P->stream;
@@ -1357,6 +1357,9 @@ int host_execute(wavemoth_plan P, bool adjoint = false) {
       rc = cuda_check(cudaMemcpyAsync(P->d_alm, alm_host, alm_bytes, cudaMemcpyHostToDevice, st),
                       "alm upload");
     rc = rc ? rc : run_alm2map(P, alm, map, st, adjoint ? 4.0 * 3.14159265358979323846 / (double)P->npix : 1.0);
+    if (adjoint && !rc && P->d_ring_weights)
+      rc = cuda_check(wm::launch_ring_weights(P->d_rings, P->ni, P->d_ring_weights, P->nmaps, map, st),
+                      "ring weights launch");
     if (!devptr && !rc)
       rc = cuda_check(cudaMemcpyAsync(map_host, P->d_map, map_bytes, cudaMemcpyDeviceToHost, st),
                       "map download");

@@ -230,6 +230,9 @@ cudaError_t launch_strided_copy(double *dst, int64_t dpitch, const double *src, 
 cudaError_t launch_ring_synthesis(const RingParams &prm, cudaStream_t st);
 // alm rows [0, split) with zero imaginary parts, the others twice (rows of nvecs doubles).
 cudaError_t launch_backward_weights(double *alm, int64_t split, int64_t rows, int32_t nvecs, cudaStream_t st);
+// The map's rings times the weights of their pairs.
+cudaError_t launch_ring_weights(const DevRing *rings, int32_t ni, const double *weights, int32_t nmaps, double *map,
+                                cudaStream_t st);
 // y += x (n doubles).
 cudaError_t launch_accumulate(const double *x, double *y, int64_t n, cudaStream_t st);
 // m-sharded plans: moves the 2 nvecs doubles of every (ring of this part,

@@ -849,6 +849,18 @@ __global__ void k_accumulate(const double *__restrict__ x, double *__restrict__ 
     y[i] += x[i];
 }
 
+// The rings of pair blockIdx.x times its weight.
+__global__ void k_ring_weights(const DevRing *__restrict__ rings, const double *__restrict__ weights, int32_t nmaps,
+                               double *__restrict__ map) {
+  const DevRing R = rings[blockIdx.x];
+  const double w = weights[blockIdx.x];
+  const int64_t n = (int64_t)R.n * nmaps;
+  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
+    map[R.off_north * nmaps + i] *= w;
+    if (R.off_south != R.off_north) map[R.off_south * nmaps + i] *= w;
+  }
+}
+
 // One warp per (ring, m) row pair: 2 nvecs doubles between the ring-side q
 // and the exchange buffer.
 __global__ void k_shard_exchange(const int64_t *__restrict__ tab, int64_t nrings, int32_t mcount, int32_t nvecs,
@@ -878,6 +890,12 @@ cudaError_t launch_backward_weights(double *alm, int64_t split, int64_t rows, in
   const int64_t n = rows * nvecs;
   if (n <= 0) return cudaSuccess;
   k_backward_weights<<<(unsigned)std::min<int64_t>((n + 255) / 256, 8192), 256, 0, st>>>(alm, split * nvecs, n);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_ring_weights(const DevRing *rings, int32_t ni, const double *weights, int32_t nmaps, double *map,
+                                cudaStream_t st) {
+  k_ring_weights<<<ni, 256, 0, st>>>(rings, weights, nmaps, map);
   return cudaGetLastError();
 }
 

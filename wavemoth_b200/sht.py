@@ -43,6 +43,7 @@ class Transform:
             raise WavemothError("plan creation failed: " + last_error())
         self._plan = p
         self._plans = {"alm2map": p, "map2alm": p}
+        self.ring_weights = None
 
     def _stream(self):
         return torch.cuda.current_stream().cuda_stream
@@ -107,15 +108,17 @@ class Transform:
 
         import numpy as np
         if weights is None:
+            w = None
             rc = _native.lib().wavemoth_plan_set_ring_weights(self._plan, None)
         else:
-            w = np.ascontiguousarray(weights, dtype=np.float64)
+            w = np.array(weights, dtype=np.float64, order="C")
             if w.shape != (2 * self.nside,):
                 raise ValueError("weights must have shape (%d,)" % (2 * self.nside))
             rc = _native.lib().wavemoth_plan_set_ring_weights(
                 self._plan, w.ctypes.data_as(ctypes.POINTER(ctypes.c_double)))
         if rc != 0:
             raise WavemothError("set_ring_weights failed: " + last_error())
+        self.ring_weights = w
 
     def device_status(self):
         """Waits for torch's current stream and raises if a kernel recorded an
