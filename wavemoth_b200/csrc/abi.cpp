@@ -1385,11 +1385,12 @@ namespace wm {
 
 // Batch coalescing (batch.cpp): two device-pointer plans compute the same
 // transform on their maps when they share the device image (file, lmax,
-// mmax, precision) and the settings that change results.
+// mmax, precision) and the settings that change results or bound their waits.
 bool plans_coalescible(wavemoth_plan a, wavemoth_plan b) {
   return a && b && a != b && a->img == b->img && a->flags == b->flags && a->lmax == b->lmax &&
-         a->mmax == b->mmax && a->phase_shifts == b->phase_shifts && !a->d_ring_weights &&
-         !b->d_ring_weights && a->nparts == 1 && b->nparts == 1 && (a->flags & WAVEMOTH_DEVICE_POINTERS);
+         a->mmax == b->mmax && a->phase_shifts == b->phase_shifts && a->wait_limit == b->wait_limit &&
+         !a->d_ring_weights && !b->d_ring_weights && a->nparts == 1 && b->nparts == 1 &&
+         (a->flags & WAVEMOTH_DEVICE_POINTERS);
 }
 
 // A device-pointer plan of `nmaps` maps on the image of P (no new image).
@@ -1399,7 +1400,10 @@ wavemoth_plan plan_with_maps(wavemoth_plan P, int nmaps) {
                               P->flags | WAVEMOTH_DEVICE_POINTERS, dense ? nullptr : P->resource_path.c_str());
   if (Q) {
     Q->phase_shifts = P->phase_shifts;
-    Q->wait_limit = P->wait_limit;
+    if (wavemoth_plan_set_wait_limit(Q, P->wait_limit)) {
+      delete Q;
+      return nullptr;
+    }
   }
   return Q;
 }
