@@ -228,7 +228,8 @@ int wavemoth_alm2map_backward_device(wavemoth_plan plan, const double *grad_map,
 /* map2alm refined by niter Jacobi iterations, a_{k+1} = a_k +
    map2alm(f - alm2map(a_k)), on device buffers (layouts as
    wavemoth_execute_map2alm_device) on `stream`.  The first call with
-   niter > 0 allocates two plan-owned buffers (a map and an alm).  With ring
+   niter > 0 allocates the plan's buffers for it (a map; split plans and files
+   with deeper trees also an alm), later calls nothing.  With ring
    weights set, every map2alm of the iteration is weighted.  New. */
 int wavemoth_map2alm_iterative_device(wavemoth_plan plan, const double *map, double *alm, int niter,
                                       void *stream);

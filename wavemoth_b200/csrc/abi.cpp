@@ -1638,7 +1638,8 @@ int wavemoth_map2alm_iterative_device(wavemoth_plan plan, const double *map, dou
   int rc = 0;
   const bool add = weighs_alm(plan);
   if (niter > 0 && !plan->d_iter_map) rc = plan->arena.alloc(&plan->d_iter_map, (size_t)nmap, "iteration map buffer");
-  if (niter > 0 && !add && !plan->d_iter_alm)
+  // (also when this call adds in place: a wait limit may change that later)
+  if (niter > 0 && (plan->split || plan->nslow > 0) && !plan->d_iter_alm)
     rc = rc ? rc : plan->arena.alloc(&plan->d_iter_alm, (size_t)nalm, "iteration alm buffer");
   if (rc) return finish(plan, rc);
   rc = run_map2alm(plan, map, alm, st);
