@@ -625,7 +625,7 @@ def run_b200(a):
                      "peak_source": "cuBLAS DGEMM 8192^3 measured by bench.py on this GPU",
                      "what": "algorithmic FP64 flops of the transform (2 per multiply-add of 64 vectors, "
                              "5 per recurrence step) over the phase time"}
-        if a.precision == "split":
+        if work["split_int8_ops_alm2map"] > 0:  # few maps of a split plan run in FP64
             ops = work["split_int8_ops_" + ("alm2map" if dominant.endswith("alm2map") else "map2alm")]
             achieved = ops / (kms[dominant] / 1e3) / 1e12
             peak = int8_peak_tops(torch)
@@ -706,7 +706,8 @@ def run_b200(a):
                    "nside": a.nside, "lmax": a.lmax, "nmaps_per_gpu": a.nmaps,
                    "precision": ("split: residual products as sliced int8 tcgen05 GEMMs (6 slices, "
                                  "products i+j<=6), FP64 recurrence/levels/rings"
-                                 if a.precision == "split" else "plain FP64"),
+                                 if a.precision == "split" and work["split_int8_ops_alm2map"] > 0 else
+                                 "split: FP64 throughout (few maps)" if a.precision == "split" else "plain FP64"),
                    "plain_fp64": plain,
                    "parity_vs_reference": parity,
                    "plan": {"eps": a.eps, "chunk": a.chunk, "memop_cost": a.memop,

@@ -303,7 +303,8 @@ int64_t wavemoth_plan_kernel_launches(wavemoth_plan plan);
    out[8] / out[9] elements of P generated by the alm2map / map2alm tiles
    per pass of 64 vectors (zero padding of the tiles included), out[10] /
    out[11] int8 tensor-core operations of one alm2map / map2alm launch
-   (residual and level GEMMs). */
+   (residual and level GEMMs); all four 0 for a plan that computes in FP64
+   (wavemoth_plan_route). */
 int wavemoth_plan_work(wavemoth_plan plan, int nmaps, double *out);
 
 /* Parses and validates a rev1 file for (Nside, lmax) exactly as plan

@@ -111,3 +111,17 @@ def test_without_room_for_the_tables():
     assert _same(_run(U, 3), _run(D, 3)) and _same(_run(T, 3), want)
     for t in (T, U, D):
         t.close()
+
+
+@pytest.mark.parametrize("precision,nmaps,polls,gemms", [("double", 3, 0, False), ("split", 3, 0, False),
+                                                         ("split", 3, 1 << 26, True), ("split", 40, 0, True),
+                                                         ("split-generate", 3, 0, True)])
+def test_reported_work_is_that_of_the_kernels_that_run(precision, nmaps, polls, gemms):
+    T = _plan(nmaps, precision)
+    if polls:
+        _limit(T, polls)
+    work = T.work()
+    for key in ("split_int8_ops_alm2map", "split_int8_ops_map2alm", "split_elems_alm2map", "split_elems_map2alm"):
+        assert (work[key] > 0) == gemms
+    assert work["legendre_flops"] > 0
+    T.close()

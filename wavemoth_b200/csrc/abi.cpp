@@ -1815,6 +1815,8 @@ int wavemoth_plan_work(wavemoth_plan plan, int nmaps, double *out) {
   out[5] = (double)G.rec_elems;
   out[6] = (double)G.dense_elems;
   out[7] = (double)plan->grid;
+  out[8] = out[9] = out[10] = out[11] = 0.0;
+  if (use_direct(plan)) return 0;
   // split path: 64-row (or 64-column) K chunks of 128-row M tiles; per K
   // step of 32, nine MMAs with N summing to 1664 (six slices, i + j <= 6)
   double ea = 0.0, eb = 0.0, la = 0.0, lb = 0.0;
