@@ -607,28 +607,40 @@ void free_host_direct(wm::HostProgram &G) {
   G.direct_tile_seeds.clear(); G.direct_tile_seeds.shrink_to_fit();
 }
 
-// Fills the plan's FP64 tables from its group columns.
+// Fills the plan's FP64 tables from its group columns.  FP64 images do not keep
+// those: they pass through the plan's q buffer, in as many parts as that needs
+// (allocating and freeing room for them took 0.7 of the 2.3 ms of a plan at nside
+// 32); a shard, which has no q buffer, allocates.
 int setup_direct(wavemoth_plan P) {
   auto &G = P->img->prog;
-  if (!G.ngcols) return 0;
+  const int64_t n = G.ngcols;
+  if (!n) return 0;
   // the uploads went through the default stream, which the plan's does not wait for
   int rc = cuda_check(cudaStreamSynchronize(0), "image upload");
-  wm::DevGCol *gcols = nullptr;
-  if (!rc && !P->d_gcols) {
-    const size_t bytes = G.gcols.size() * sizeof(wm::DevGCol);
-    rc = cuda_check(cudaMalloc(&gcols, bytes), "group columns");
-    if (!rc)
-      rc = cuda_check(cudaMemcpyAsync(gcols, G.gcols.data(), bytes, cudaMemcpyHostToDevice, P->stream),
-                      "group columns");
+  wm::DevGCol *gcols = P->d_gcols, *own = nullptr;
+  int64_t part = n;
+  if (!gcols && P->nparts == 1) {
+    gcols = reinterpret_cast<wm::DevGCol *>(P->d_q);
+    const int64_t q_bytes = 2LL * (P->mmax + 1) * P->ni * P->nvecs * (int64_t)sizeof(double);
+    part = std::min<int64_t>(n, q_bytes / (int64_t)sizeof(wm::DevGCol));
+  } else if (!gcols) {
+    rc = rc ? rc : cuda_check(cudaMalloc(&own, n * sizeof(wm::DevGCol)), "group columns");
+    gcols = own;
   }
   if (!rc)
     rc = cuda_check(cudaMemsetAsync(P->d_direct_seeds, 0, std::max<int64_t>(G.direct_seeds, 1) * sizeof(double2),
                                     P->stream), "segment seeds");
-  if (!rc)
-    rc = cuda_check(wm::launch_direct_setup(direct_params(P), gcols ? gcols : P->d_gcols, P->d_f64, P->d_direct_cols,
-                                            P->d_direct_inj, P->d_direct_seeds, P->stream), "column setup launch");
+  for (int64_t first = 0; first < n && !rc; first += part) {
+    const int64_t count = std::min(part, n - first);
+    if (!P->d_gcols)
+      rc = cuda_check(cudaMemcpyAsync(gcols, G.gcols.data() + first, count * sizeof(wm::DevGCol),
+                                      cudaMemcpyHostToDevice, P->stream), "group columns");
+    if (!rc)
+      rc = cuda_check(wm::launch_direct_setup(direct_params(P), gcols, first, count, P->d_f64, P->d_direct_cols,
+                                              P->d_direct_inj, P->d_direct_seeds, P->stream), "column setup launch");
+  }
   if (!rc) rc = cuda_check(cudaStreamSynchronize(P->stream), "column setup");
-  cudaFree(gcols);
+  cudaFree(own);
   return rc;
 }
 

@@ -92,9 +92,10 @@ struct DirectParams {
 cudaError_t launch_direct_a2m(DirectParams prm, const DevDirectTileA *const (&tiles)[2], const int32_t (&ntiles)[2],
                               int sms, int max_ctas, cudaStream_t st);
 cudaError_t launch_direct_m2a(const DirectParams &prm, int max_ctas, cudaStream_t st);
-// Plan creation: cols, inj and seeds (zeroed by the caller) of every group column.
-cudaError_t launch_direct_setup(const DirectParams &prm, const DevGCol *gcols, const double *f64, DevDirectCol *cols,
-                                double *inj, double2 *seeds, cudaStream_t st);
+// Plan creation: cols, inj and seeds (zeroed by the caller) of n group columns
+// from the first-th, which gcols holds.
+cudaError_t launch_direct_setup(const DirectParams &prm, const DevGCol *gcols, int64_t first, int64_t n,
+                                const double *f64, DevDirectCol *cols, double *inj, double2 *seeds, cudaStream_t st);
 
 // Split-precision residual path (legendre_split.cu).
 struct SplitParams {

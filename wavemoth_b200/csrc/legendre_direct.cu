@@ -423,13 +423,13 @@ __global__ void __launch_bounds__(kDirectThr, NT == 2 ? 3 : 4) k_direct_m2a(Dire
 }
 
 // ------------------------------------------------------------------------
-// Plan creation: column data, first values and segment seeds of every group
-// column, from the plan's strips and the row scales.
+// Plan creation: column data, first values and segment seeds of group columns
+// first .. first + n - 1 (gcols: those), from the plan's strips and the row scales.
 // ------------------------------------------------------------------------
-__global__ void k_direct_setup(DirectParams p, const DevGCol *gcols, const double *f64, DevDirectCol *cols, double *inj,
-                               double2 *seeds) {
-  const int64_t gc = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gc >= p.ngcols) return;
+__global__ void k_direct_setup(DirectParams p, const DevGCol *gcols, int64_t first, int64_t n, const double *f64,
+                               DevDirectCol *cols, double *inj, double2 *seeds) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, gc = first + i;
+  if (i >= n) return;
   int lo = 0, hi = p.ngroups - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) / 2;
@@ -437,7 +437,7 @@ __global__ void k_direct_setup(DirectParams p, const DevGCol *gcols, const doubl
     else hi = mid - 1;
   }
   const DevGroup G = p.groups[lo];
-  const DevGCol C = gcols[gc];
+  const DevGCol C = gcols[i];
   const int R = G.nrows, c = (int)(gc - G.cols);
   const double2 *ab = p.ab + G.coef;
   const double *scale = p.scale + G.coef;
@@ -515,10 +515,10 @@ cudaError_t launch_direct_m2a(const DirectParams &p, int max_ctas, cudaStream_t 
   return launch_overlapped(wide ? k_direct_m2a<2> : k_direct_m2a<1>, grid, kDirectThr, 0, st, p, npass);
 }
 
-cudaError_t launch_direct_setup(const DirectParams &p, const DevGCol *gcols, const double *f64, DevDirectCol *cols,
-                                double *inj, double2 *seeds, cudaStream_t st) {
-  if (p.ngcols == 0) return cudaSuccess;
-  k_direct_setup<<<(unsigned)((p.ngcols + 127) / 128), 128, 0, st>>>(p, gcols, f64, cols, inj, seeds);
+cudaError_t launch_direct_setup(const DirectParams &p, const DevGCol *gcols, int64_t first, int64_t n,
+                                const double *f64, DevDirectCol *cols, double *inj, double2 *seeds, cudaStream_t st) {
+  if (n <= 0) return cudaSuccess;
+  k_direct_setup<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(p, gcols, first, n, f64, cols, inj, seeds);
   return cudaGetLastError();
 }
 

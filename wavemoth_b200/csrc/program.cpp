@@ -848,6 +848,9 @@ bool build_fast_path(HostProgram &P, bool split, std::string &err) {
   P.xrows = 0;
   P.max_root_k = 0;
   P.max_root_n = 0;
+  size_t ncols = 0;
+  for (const DevDBlock &D : P.dblocks) ncols += (size_t)D.ncols;
+  P.gcols.reserve(ncols);
   for (size_t mi = 0; mi < P.mats.size(); ++mi) {
     DevMatrix &M = P.mats[mi];
     M.fast = 0;
@@ -965,7 +968,7 @@ bool build_fast_path(HostProgram &P, bool split, std::string &err) {
   std::stable_sort(P.direct_b.begin(), P.direct_b.end(), [](const DevDirectTileB &a, const DevDirectTileB &b) {
     return (int64_t)a.nact * a.seg > (int64_t)b.nact * b.seg;
   });
-  build_split_tables(P);
+  if (split) build_split_tables(P);
   return true;
 }
 
