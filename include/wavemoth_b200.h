@@ -31,7 +31,7 @@ extern "C" {
 #define WAVEMOTH_SPLIT_GENERATE 0x400    /* with WAVEMOTH_PRECISION_SPLIT: generate the residual P
                                             inside the GEMM kernels at every call instead of
                                             slicing it once per plan into device memory (6 bytes
-                                            per element of the residual tiles, about 20 GB at
+                                            per element of the residual tiles, about 18 GB at
                                             nside 1024); the plan also falls back to this when
                                             the device lacks the memory.  Same results as the
                                             GEMMs on stored slices.  Plans of few maps stay on
@@ -244,7 +244,7 @@ int wavemoth_map2alm_iterative_device(wavemoth_plan plan, const double *map, dou
    direction (src/wavemoth.c:1271-1283 is synthesis only). */
 void wavemoth_execute_adjoint(wavemoth_plan plan);
 
-/* Caps the SMs the plan's persistent Legendre kernels (the tensor-core and
+/* Caps the SMs the plan's Legendre kernels (the FP64 kernels and the
    split GEMMs, which walk the plan's (m, parity) tile list) may occupy; 0
    restores all.  Used by the batch scheduler so that concurrent requests
    share the GPU; results do not depend on it. */

@@ -81,7 +81,7 @@ struct ImageRefs {
   double *d_f64 = nullptr;
   int32_t *d_i32 = nullptr;
   int32_t *d_order = nullptr;       // all matrices, largest first (generic kernel over everything)
-  int32_t *d_order_slow = nullptr;  // matrices left to the generic kernel by the tensor-core path
+  int32_t *d_order_slow = nullptr;  // matrices left to the generic kernel (build_fast_path)
   int32_t nslow = 0;
   // row groups
   wm::DevGroup *d_groups = nullptr;
@@ -456,6 +456,11 @@ wm::SplitParams split_params(wavemoth_plan P) {
 // lmax 1500: 3 maps 2841 / 7254, 8 maps 5474 / 7532, 16 maps 10660 / 7838.  Plans
 // that are to generate P rather than hold it would hold the FP64 tables instead,
 // and keep the GEMMs.
+// kDirectMinElems is not where the times cross.  FP64 is the faster one below it
+// as well (1 / 4 / 14 maps: nside 32, lmax 64 21 / 23 / 27 us against 50 / 51 / 55;
+// nside 64, lmax 191 31 / 37 / 73 against 78 / 83 / 97; nside 96, lmax 192 39 / 50 /
+// 116 against 105 / 111 / 165); the bound leaves split plans of small files the
+// kernels, and the bits, that they have always had.
 constexpr int64_t kDirectMinElems = 4 << 20;
 
 bool prefers_direct(wavemoth_plan P) {

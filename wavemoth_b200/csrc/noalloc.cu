@@ -7,8 +7,8 @@
 // critical.  wavemoth_legendre_alm2map_noalloc runs the generic FP64
 // butterfly Legendre kernel (k_alm2map_legendre, SIMT, persistent CTAs on a
 // work queue) over every (m, parity) matrix of the plan; the plan's own path
-// runs that kernel only for trees of depth >= 2 and the FP64 tensor-core
-// kernels for the rest, so the two agree to rounding, not bitwise.  Its
+// runs that kernel only for trees of depth >= 2 and the kernels of the row
+// groups for the rest, so the two agree to rounding, not bitwise.  Its
 // per-CTA level buffers and its work-queue counter come from the
 // file-scope device array below instead of plan-allocated scratch.  The
 // caller passes the input (alm) and the output (q) as device pointers; the

@@ -72,7 +72,7 @@ struct DevMatrix {
   int64_t root_map;      // i32 arena, 2 per depth-0 row: (strip index, column within the strip)
   double cost;           // estimated work, for scheduling
   int64_t xrow;          // first row of this matrix in the X buffer (depth-1 matrices), else -1
-  int32_t fast;          // 1: handled by the tensor-core path (depth <= 1)
+  int32_t fast;          // 1: its residual blocks form row groups (depth <= 1), 0: generic kernels
   int32_t pad2;
 };
 

@@ -573,8 +573,8 @@ bool compile_resource(const char *data, size_t len, int nside_expect, int lmax_e
 
 namespace wm {
 
-// Row groups, column tables, work units and seed bookkeeping of the
-// tensor-core path (plan.h).  Matrices of depth 0 (one residual block over
+// Row groups, column tables, work units and seed bookkeeping of the FP64
+// and split paths (plan.h).  Matrices of depth 0 (one residual block over
 // all rows) and depth 1 (every root a (T, B) pair over two leaves, T blocks
 // on rows [0, nk/2), B blocks on [nk/2, nk) -- butterfly.pyx:570-573) are
 // taken; anything else stays with the generic kernels.
@@ -946,7 +946,7 @@ bool build_fast_path(HostProgram &P, bool split, std::string &err) {
       }
       G.ncols = (int32_t)(P.gcols.size() - G.cols);
       // columns by first active row, so that the column tiles of the
-      // tensor-core kernels span similar row ranges
+      // kernels span similar row ranges
       std::stable_sort(P.gcols.begin() + G.cols, P.gcols.end(),
                        [](const DevGCol &a, const DevGCol &b) { return a.start < b.start; });
       G.nchunks = (G.nrows + kSeedRows - 1) / kSeedRows;

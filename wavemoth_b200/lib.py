@@ -19,9 +19,9 @@ WAVEMOTH_DEVICE_POINTERS = 0x100
 WAVEMOTH_PRECISION_SPLIT = 0x200
 WAVEMOTH_SPLIT_GENERATE = 0x400
 WAVEMOTH_DENSE = 0x800
-# precision= of the plans: FP64 tensor cores, or the split int8 path with the
-# residual P sliced once per plan ("split") or generated at every call
-# ("split-generate", less device memory)
+# precision= of the plans: FP64 units, or the split int8 path with the residual P
+# sliced once per image ("split"; plans of few maps run in FP64 where that is
+# faster) or generated at every call ("split-generate", less device memory)
 PRECISION_FLAGS = {"double": 0, "split": WAVEMOTH_PRECISION_SPLIT,
                    "split-generate": WAVEMOTH_PRECISION_SPLIT | WAVEMOTH_SPLIT_GENERATE}
 

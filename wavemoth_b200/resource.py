@@ -577,7 +577,7 @@ class ResourceComputer:
         self.check_stability = check_stability
         # None: every depth the tree has (the reference's choice); else the
         # level choice stops at this many interpolation levels -- 1 keeps
-        # every matrix on this library's tensor-core paths, which run trees
+        # every matrix on this library's fast paths, which run trees
         # of depth 0 and 1 (deeper ones run on the generic FP64 kernels)
         self.max_levels = max_levels
 
