@@ -848,14 +848,17 @@ bool build_fast_path(HostProgram &P, bool split, std::string &err) {
   P.xrows = 0;
   P.max_root_k = 0;
   P.max_root_n = 0;
+  auto elsewhere = [&](const DevMatrix &M) { return P.shard_m1 >= 0 && (M.m < P.shard_m0 || M.m >= P.shard_m1); };
   size_t ncols = 0;
-  for (const DevDBlock &D : P.dblocks) ncols += (size_t)D.ncols;
+  for (const DevMatrix &M : P.mats)
+    for (int b = M.dblock_begin; b < M.dblock_end && M.nlevels <= 1 && !elsewhere(M); ++b)
+      ncols += (size_t)P.dblocks[b].ncols;
   P.gcols.reserve(ncols);
   for (size_t mi = 0; mi < P.mats.size(); ++mi) {
     DevMatrix &M = P.mats[mi];
     M.fast = 0;
     M.xrow = -1;
-    if (P.shard_m1 >= 0 && (M.m < P.shard_m0 || M.m >= P.shard_m1)) continue;  // another shard's
+    if (elsewhere(M)) continue;  // another shard's
     const int nblk = M.dblock_end - M.dblock_begin;
     bool ok = M.nlevels == 0 || M.nlevels == 1;
     if (ok && M.nlevels == 0) ok = (nblk == 1);
