@@ -833,6 +833,17 @@ static void direct_tiles(HostProgram &P, DevGroup &G, int32_t gi) {
   }
 }
 
+// Columns of the blocks of this shard's matrices of depth 0 and 1: what the
+// groups can have.
+static size_t group_columns(const HostProgram &P) {
+  size_t n = 0;
+  for (const DevMatrix &M : P.mats) {
+    if (M.nlevels > 1 || (P.shard_m1 >= 0 && (M.m < P.shard_m0 || M.m >= P.shard_m1))) continue;
+    for (int b = M.dblock_begin; b < M.dblock_end; ++b) n += (size_t)P.dblocks[b].ncols;
+  }
+  return n;
+}
+
 bool build_fast_path(HostProgram &P, bool split, std::string &err) {
   P.groups.clear();
   P.gcols.clear();
@@ -848,17 +859,12 @@ bool build_fast_path(HostProgram &P, bool split, std::string &err) {
   P.xrows = 0;
   P.max_root_k = 0;
   P.max_root_n = 0;
-  auto elsewhere = [&](const DevMatrix &M) { return P.shard_m1 >= 0 && (M.m < P.shard_m0 || M.m >= P.shard_m1); };
-  size_t ncols = 0;
-  for (const DevMatrix &M : P.mats)
-    for (int b = M.dblock_begin; b < M.dblock_end && M.nlevels <= 1 && !elsewhere(M); ++b)
-      ncols += (size_t)P.dblocks[b].ncols;
-  P.gcols.reserve(ncols);
+  P.gcols.reserve(group_columns(P));
   for (size_t mi = 0; mi < P.mats.size(); ++mi) {
     DevMatrix &M = P.mats[mi];
     M.fast = 0;
     M.xrow = -1;
-    if (elsewhere(M)) continue;  // another shard's
+    if (P.shard_m1 >= 0 && (M.m < P.shard_m0 || M.m >= P.shard_m1)) continue;  // another shard's
     const int nblk = M.dblock_end - M.dblock_begin;
     bool ok = M.nlevels == 0 || M.nlevels == 1;
     if (ok && M.nlevels == 0) ok = (nblk == 1);
