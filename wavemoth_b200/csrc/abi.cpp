@@ -1347,7 +1347,8 @@ int finish(wavemoth_plan P, int rc) {
 // shard does not have (its q buffers are the caller's).
 int whole_plan_check(wavemoth_plan P, const void *a, const void *b) {
   if (!P || !a || !b) return set_error(WAVEMOTH_ERR_ARG, "NULL plan or buffer");
-  if (P->nparts > 1) return set_error(WAVEMOTH_ERR_ARG, "a shard of a plan runs through the wavemoth_shard_ calls only");
+  if (P->nparts > 1)
+    return set_error(WAVEMOTH_ERR_ARG, "a shard of a plan runs through the wavemoth_shard_ calls only");
   return 0;
 }
 
